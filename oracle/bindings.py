@@ -31,6 +31,12 @@ REF_GPU_SO = os.path.join(HERE, "_ref", "libptref_gpu.so")
 # libraries under oracle/_ref are used where the tree is absent).
 REF_ROOT = os.environ.get("LSYSTEM_REFERENCE_ROOT", "/root/reference")
 
+
+def _ref_tree() -> bool:
+    """The reference's sources are there (an empty directory in their place counts as absent)."""
+    return os.path.isdir(os.path.join(REF_ROOT, "PathTracerLib"))
+
+
 _fp = C.POINTER(C.c_float)
 _dp = C.POINTER(C.c_double)
 _u32p = C.POINTER(C.c_uint32)
@@ -68,9 +74,9 @@ def build_oracle(force: bool = False) -> str:
 
 def build_ref() -> Optional[str]:
     """Compiles the reference's own sources for the host where the reference tree exists."""
-    if os.path.exists(REF_SO) and not os.path.isdir(REF_ROOT):
+    if os.path.exists(REF_SO) and not _ref_tree():
         return REF_SO
-    if not os.path.isdir(REF_ROOT):
+    if not _ref_tree():
         return None
     src = [os.path.join(HERE, "ref_harness.cpp"), os.path.join(HERE, "ref_shim", "curand_kernel.h")]
     if not os.path.exists(REF_SO) or any(os.path.getmtime(s) > os.path.getmtime(REF_SO) for s in src):
@@ -80,7 +86,7 @@ def build_ref() -> Optional[str]:
 
 def build_ref_gpu() -> Optional[str]:
     """Compiles the reference's CUDA render kernels for sm_100a where the reference tree exists."""
-    if not os.path.isdir(REF_ROOT):
+    if not _ref_tree():
         return REF_GPU_SO if os.path.exists(REF_GPU_SO) else None
     src = [os.path.join(HERE, "ref_gpu_harness.cu"), os.path.join(HERE, "Makefile")]
     if not os.path.exists(REF_GPU_SO) or any(os.path.getmtime(s) > os.path.getmtime(REF_GPU_SO) for s in src):
@@ -94,7 +100,7 @@ WRAPPER_BIN = os.path.join(HERE, "_ref", "wrapper_check")
 
 def build_ref_gen() -> Optional[str]:
     """Compiles the reference's scene generator (LSystemLib, Turtle.cpp, Spline.cpp) for the host."""
-    if not os.path.isdir(REF_ROOT):
+    if not _ref_tree():
         return REF_GEN_SO if os.path.exists(REF_GEN_SO) else None
     src = [os.path.join(HERE, "ref_gen_harness.cpp"), os.path.join(HERE, "Makefile")]
     if not os.path.exists(REF_GEN_SO) or any(os.path.getmtime(s) > os.path.getmtime(REF_GEN_SO) for s in src):
@@ -104,7 +110,7 @@ def build_ref_gen() -> Optional[str]:
 
 def build_wrapper() -> Optional[str]:
     """Compiles the C++ PathTracer-shaped wrapper (tests/cpp) against the reference's headers."""
-    if not os.path.isdir(REF_ROOT):
+    if not _ref_tree():
         return WRAPPER_BIN if os.path.exists(WRAPPER_BIN) else None
     root = os.path.dirname(HERE)
     src = [os.path.join(root, "tests", "cpp", f) for f in ("wrapper_check.cpp", "PathTracerB200.h")] + \
