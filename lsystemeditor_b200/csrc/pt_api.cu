@@ -1264,7 +1264,8 @@ bool ensureBounceGraphs(pt_renderer* r, const LaunchCtx* c, bool inst, int nw)
             (static_cast<unsigned long long>(r->extendLane ? 1 : 0) << 8) |
             (static_cast<unsigned long long>(r->gridExtendLane) << 9) |
             (static_cast<unsigned long long>(r->gridShadowLane) << 22) |
-            (static_cast<unsigned long long>(r->gridShadeMiss) << 36),
+            (static_cast<unsigned long long>(r->gridShadeMiss) << 36) |
+            (static_cast<unsigned long long>(r->scenes.size() > 1 ? 1 : 0) << 62),
         reinterpret_cast<unsigned long long>(r->stream)};
     if (r->bounceGraph[0] != nullptr && std::equal(key, key + 6, r->bounceKey)) {
         return true;
@@ -1283,10 +1284,10 @@ bool ensureBounceGraphs(pt_renderer* r, const LaunchCtx* c, bool inst, int nw)
         }
         int sel = 0;
         for (int it = 0; it < 4; ++it) {
-            launchExtend(c, sel, g == 0 && it == 0, it, extendGrid(r, false, inst), false, inst, r->extendLane, s);
+            launchExtend(c, sel, g == 0 && it == 0, it, extendGrid(r, false, inst), false, inst, r->extendLane, r->scenes.size() > 1, s);
             launchShadeMiss(c, it, sel, r->gridShadeMiss, nw, s);
             launchShade(c, sel, it, shadeGrid(r, nw), nw, s);
-            launchShadow(c, it, shadowGrid(r, false, inst), false, inst, r->extendLane, s);
+            launchShadow(c, it, shadowGrid(r, false, inst), false, inst, r->extendLane, r->scenes.size() > 1, s);
             launchFinalize(c, sel, r->gridShadow, nw, s);
             if (slotOrdered(r)) {
                 launchNextQueue(c, sel, r->gridShadow, s);
@@ -1746,7 +1747,7 @@ int pt_render(pt_renderer* r, int waves)
                 const int iter = static_cast<int>(it & 0x7fffffff);
                 {
                     StageTimer tm(r, kExtend);
-                    launchExtend(c, sel, it == 0, iter, extendGrid(r, countVisits, inst), countVisits, inst, r->extendLane, s);
+                    launchExtend(c, sel, it == 0, iter, extendGrid(r, countVisits, inst), countVisits, inst, r->extendLane, r->scenes.size() > 1, s);
                 }
                 {
                     StageTimer tm(r, kShade);
@@ -1755,7 +1756,7 @@ int pt_render(pt_renderer* r, int waves)
                 }
                 {
                     StageTimer tm(r, kShadow);
-                    launchShadow(c, iter, shadowGrid(r, countVisits, inst), countVisits, inst, r->extendLane, s);
+                    launchShadow(c, iter, shadowGrid(r, countVisits, inst), countVisits, inst, r->extendLane, r->scenes.size() > 1, s);
                 }
                 {
                     StageTimer tm(r, kFinalize);

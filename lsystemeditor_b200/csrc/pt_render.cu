@@ -33,7 +33,7 @@
 #include "pt_bsdf.cuh"
 #include "pt_path.cuh"
 #include "pt_spectral.cuh"
-#include "pt_trace.cuh"
+#include "pt_traverse.cuh"
 
 #include <atomic>
 #include <cooperative_groups.h>
@@ -623,6 +623,7 @@ __global__ void __launch_bounds__(256) k_generate(const LaunchCtx* __restrict__ 
         c.q.counts[5] = 0u;
         c.q.counts[8] = 0u;  // fetch counters of the first extend and shadow stages
         c.q.counts[10] = 0u;
+        c.q.counts[12] = 0u; // Q1 mark of the first extend stage
     }
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
         initPath<NW>(c, static_cast<uint32_t>(i), jobOffset + static_cast<unsigned long long>(i));
@@ -698,401 +699,25 @@ __global__ void __launch_bounds__(256, PT_EXTEND_MIN_BLOCKS) k_extend(const Laun
     }
 }
 
-#ifndef PT_EXTEND_LANE_THREADS
-#define PT_EXTEND_LANE_THREADS 256
-#endif
 #ifndef PT_EXTEND_LANE_MIN_BLOCKS
-#define PT_EXTEND_LANE_MIN_BLOCKS 3
+#define PT_EXTEND_LANE_MIN_BLOCKS 6
 #endif
 #ifndef PT_SHADOW_LANE_MIN_BLOCKS
-#define PT_SHADOW_LANE_MIN_BLOCKS 4
-#endif
-#ifndef PT_EXTEND_LANE_SYNC
-#define PT_EXTEND_LANE_SYNC false
-#endif
-#ifndef PT_SHADOW_LANE_SYNC
-#define PT_SHADOW_LANE_SYNC false
-#endif
-#ifndef PT_SHADOW_LANE
-#define PT_SHADOW_LANE 1
+#define PT_SHADOW_LANE_MIN_BLOCKS 7
 #endif
 
-// A ray of the per-lane traversal: its scene, origin, normalised direction and
-// the parametric interval it is tested on.
-struct LaneRay {
-    const DevScene* S;
-    float3 o;
-    float3 dn;
-    float tMin;
-    float tMax;
-};
-
-// Per-lane ray replacement (Aila & Laine 2009, "dynamic fetch") over a queue of
-// `count` rays of flat scenes: a lane whose ray is finished takes the next
-// queue entry at once, while the other lanes of its warp go on traversing, so
-// a warp is not held by its longest ray.  One loop iteration is one step of
-// traceRay's traversal (a node's children, then the triangles of that node),
-// with the same postponing, stacks and tie rule, so the results are
-// traceRay's.  Two loop forms:
-//   Sync = false: a lane fetches as soon as it is idle (the idle lanes of the
-//     moment share one atomic) and the lanes of a warp are not reconverged, so
-//     the scheduler can issue from the lanes that fetch while the others wait
-//     on node loads.  This form is the faster of the two on the 972k-triangle
-//     tree (closest hit) and on the 64-tree batch (shadow rays).
-//   Sync = true: every iteration is warp-synchronous (one ballot fetch for the
-//     idle lanes at the top, a full-warp vote to leave), so the lanes of a
-//     warp step together.
-//   load(k, ray) -> bool: reads queue entry k into `ray`; false when the entry
-//     was decided without the wide traversal (and its result written).
-//   finish(k, hit, t, u, v, tri): the result of entry k (tri = original
-//     triangle index; for AnyHit, hit means occluded and t, u, v, tri are unset).
-// Rays finish in no particular order.
-template <bool AnyHit, bool Sync, class Load, class Finish>
-__device__ __forceinline__ void laneTraversal(unsigned int count, unsigned int* fetch, uint2* sstack, int sstride,
-    unsigned int* overflowCounter, Load load, Finish finish)
-{
-    uint2 stack[kTraversalStack];
-    bool active = false;
-    unsigned int k = 0;
-    LaneRay r{nullptr, f3(0.0f, 0.0f, 0.0f), f3(0.0f, 0.0f, 0.0f), 0.0f, 0.0f};
-    float3 idir = r.o;
-    uint32_t octinv = 0;
-    uint2 ngroup = make_uint2(0u, 0u), tgroup = make_uint2(0u, 0u);
-    int sp = 0;
-    float closest = kRayTMax;
-    uint32_t best = 0xFFFFFFFFu;
-    float bu = 0.0f, bv = 0.0f;
-    bool overflow = false;
-
-    auto push = [&](uint2 g) -> bool {
-        if (sp < kSharedStack) {
-            sstack[sp * sstride] = g;
-        } else if (sp < kSharedStack + kTraversalStack) {
-            stack[sp - kSharedStack] = g;
-        } else {
-            return false;
-        }
-        ++sp;
-        return true;
-    };
-    auto done = [&](bool hit) {
-        finish(k, hit, closest, bu, bv, hit && !AnyHit ? leafId(r.S->tris, best) : 0xFFFFFFFFu);
-        if (overflow && overflowCounter != nullptr && !(AnyHit && hit)) {
-            atomicAdd(overflowCounter, 1u); // rays whose stack overflowed, as traceRay counts them (an occluded any-hit ray is not counted)
-        }
-        overflow = false;
-        active = false;
-    };
-    auto begin = [&]() {
-        idir = f3(__frcp_rn(r.dn.x), __frcp_rn(r.dn.y), __frcp_rn(r.dn.z));
-        const uint32_t oct = (r.dn.x < 0.0f ? 4u : 0u) | (r.dn.y < 0.0f ? 2u : 0u) | (r.dn.z < 0.0f ? 1u : 0u);
-        octinv = 7u - oct;
-        ngroup = make_uint2(0u, 0x80000000u | (1u << oct));
-        tgroup = make_uint2(0u, 0u);
-        sp = 0;
-        closest = r.tMax;
-        best = 0xFFFFFFFFu;
-        bu = bv = 0.0f;
-        active = true;
-    };
-    const unsigned int lane = threadIdx.x & 31u;
-    bool drained = false;
-    for (;;) {
-        if constexpr (Sync) {
-            const bool want = !active && !drained;
-            const unsigned int wantMask = __ballot_sync(0xFFFFFFFFu, want);
-            if (wantMask != 0u) {
-                const int leader = __ffs(wantMask) - 1;
-                unsigned int base = 0;
-                if (static_cast<int>(lane) == leader) {
-                    base = atomicAdd(fetch, static_cast<unsigned int>(__popc(wantMask)));
-                }
-                base = __shfl_sync(0xFFFFFFFFu, base, leader);
-                if (want) {
-                    k = base + __popc(wantMask & ((1u << lane) - 1u));
-                    if (k >= count) {
-                        drained = true; // the queue is drained
-                    } else if (load(k, r)) {
-                        begin();
-                    }
-                    // (an entry decided by load leaves the lane idle: it fetches again)
-                }
-            }
-            if (!__any_sync(0xFFFFFFFFu, active || !drained)) {
-                break;
-            }
-        } else if (!active) {
-            // the lanes without a ray take the next queue entries together (one atomic)
-            cg::coalesced_group g = cg::coalesced_threads();
-            unsigned int base = 0;
-            if (g.thread_rank() == 0) {
-                base = atomicAdd(fetch, g.size());
-            }
-            k = g.shfl(base, 0) + g.thread_rank();
-            if (k >= count) {
-                break; // the queue is drained
-            }
-            if (!load(k, r)) {
-                continue; // decided without the wide traversal
-            }
-            begin();
-        }
-        if (active) {
-            // one traversal step (traceRay's loop body)
-            if (ngroup.y > 0x00FFFFFFu) {
-                const uint32_t bit = 31u - __clz(ngroup.y);
-                ngroup.y &= ~(1u << bit);
-                const uint32_t slot = (bit - 24u) ^ octinv;
-                const uint32_t child = ngroup.x + __popc(ngroup.y & 0xffu & ((1u << slot) - 1u));
-                if (ngroup.y > 0x00FFFFFFu && !push(ngroup)) {
-                    overflow = true;
-                }
-                uint32_t childBase, triBase, imask;
-                const uint32_t hits =
-                    intersectChildren(r.S->nodes, child, r.o, idir, octinv, r.tMin, closest, childBase, triBase, imask);
-                ngroup = make_uint2(childBase, (hits & 0xFF000000u) | imask);
-                tgroup = make_uint2(triBase, hits & 0x00FFFFFFu);
-            } else {
-                tgroup = ngroup;
-                ngroup = make_uint2(0u, 0u);
-            }
-            bool occluded = false;
-            while (tgroup.y != 0u) {
-                if (ngroup.y > 0x00FFFFFFu && __popc(__activemask()) < kPostponeLanes && push(tgroup)) {
-                    break;
-                }
-                const int kt = __ffs(tgroup.y) - 1;
-                tgroup.y &= tgroup.y - 1u;
-                const TriVerts tv = r.S->tris[tgroup.x + kt];
-                float t, u, v;
-                if (intersectTriExact(r.o, r.dn, f3(tv.v0.x, tv.v0.y, tv.v0.z), f3(tv.v1.x, tv.v1.y, tv.v1.z),
-                        f3(tv.v2.x, tv.v2.y, tv.v2.z), r.tMin, closest, t, u, v)) {
-                    if (AnyHit) {
-                        if (t < r.tMax) {
-                            occluded = true; // traceRay's any-hit: the first hit below tMax ends the ray
-                            break;
-                        }
-                    } else if (t < closest || best == 0xFFFFFFFFu ||
-                               leafId(r.S->tris, tgroup.x + kt) > leafId(r.S->tris, best)) {
-                        closest = t; // (traceRay's tie rule: the higher original triangle index)
-                        best = tgroup.x + kt;
-                        bu = u;
-                        bv = v;
-                    }
-                }
-            }
-            if (occluded) {
-                done(true);
-            } else if (ngroup.y <= 0x00FFFFFFu) {
-                if (sp == 0) {
-                    // the ray is finished
-                    done(!AnyHit && best != 0xFFFFFFFFu && closest < r.tMax);
-                } else {
-                    --sp;
-                    ngroup = sp < kSharedStack ? sstack[sp * sstride] : stack[sp - kSharedStack];
-                }
-            }
-        }
-    }
-}
-
-// Per-lane ray replacement over the two-level BVH of an instanced scene: the
-// free-running loop of laneTraversal around traceInstanced's step (top-level
-// leaves are instances; on reaching one the ray goes to the object's space on
-// the same stack above the top level's entries, and comes back when those are
-// used up), with traceInstanced's postponing, overflow and tie rule, so the
-// results are traceInstanced's.  finish(k, hit, t, u, v, tri, inst): tri is
-// the shading-record index (object base + object triangle), inst the instance.
-template <bool AnyHit, class Load, class Finish>
-__device__ __forceinline__ void laneTraversalInst(unsigned int count, unsigned int* fetch, uint2* sstack, int sstride,
-    unsigned int* overflowCounter, Load load, Finish finish)
-{
-    uint2 stack[kTraversalStack];
-    bool active = false;
-    unsigned int k = 0;
-    LaneRay r{nullptr, f3(0.0f, 0.0f, 0.0f), f3(0.0f, 0.0f, 0.0f), 0.0f, 0.0f};
-    float3 ro = r.o, rd = r.o, idir = r.o;
-    uint32_t oct = 0, octinv = 7;
-    const CwNode* nodes = nullptr;
-    const TriVerts* leaves = nullptr;
-    int level = 0, base = 0;
-    uint32_t curInst = 0, curTriBase = 0;
-    uint2 ngroup = make_uint2(0u, 0u), tgroup = make_uint2(0u, 0u);
-    int sp = 0;
-    float closest = kRayTMax;
-    unsigned long long bestKey = ~0ull;
-    uint32_t bestTri = 0xFFFFFFFFu, bestInst = 0xFFFFFFFFu;
-    float bu = 0.0f, bv = 0.0f;
-    bool overflow = false;
-
-    auto setRay = [&](float3 a, float3 d) {
-        ro = a;
-        const float dx = fabsf(d.x) < 1.0e-20f ? copysignf(1.0e-20f, d.x) : d.x;
-        const float dy = fabsf(d.y) < 1.0e-20f ? copysignf(1.0e-20f, d.y) : d.y;
-        const float dz = fabsf(d.z) < 1.0e-20f ? copysignf(1.0e-20f, d.z) : d.z;
-        idir = f3(__frcp_rn(dx), __frcp_rn(dy), __frcp_rn(dz));
-        oct = (d.x < 0.0f ? 4u : 0u) | (d.y < 0.0f ? 2u : 0u) | (d.z < 0.0f ? 1u : 0u);
-        octinv = 7u - oct;
-    };
-    auto push = [&](uint2 g) -> bool {
-        if (sp < kSharedStack) {
-            sstack[sp * sstride] = g;
-        } else if (sp < kSharedStack + kTraversalStack) {
-            stack[sp - kSharedStack] = g;
-        } else {
-            return false;
-        }
-        ++sp;
-        return true;
-    };
-    auto done = [&](bool hit) {
-        finish(k, hit, closest, bu, bv, bestTri, bestInst);
-        if (overflow && overflowCounter != nullptr && !(AnyHit && hit)) {
-            atomicAdd(overflowCounter, 1u); // rays whose stack overflowed, as traceInstanced counts them
-        }
-        overflow = false;
-        active = false;
-    };
-    for (;;) {
-        if (!active) {
-            // the lanes without a ray take the next queue entries together (one atomic)
-            cg::coalesced_group g = cg::coalesced_threads();
-            unsigned int b = 0;
-            if (g.thread_rank() == 0) {
-                b = atomicAdd(fetch, g.size());
-            }
-            k = g.shfl(b, 0) + g.thread_rank();
-            if (k >= count) {
-                break; // the queue is drained
-            }
-            if (!load(k, r)) {
-                continue; // decided without the wide traversal
-            }
-            setRay(r.o, r.dn);
-            rd = r.dn;
-            nodes = r.S->tlasNodes;
-            leaves = r.S->tlasLeaves;
-            level = 0;
-            base = 0;
-            curInst = 0;
-            curTriBase = 0;
-            ngroup = make_uint2(0u, 0x80000000u | (1u << oct));
-            tgroup = make_uint2(0u, 0u);
-            sp = 0;
-            closest = r.tMax;
-            bestKey = ~0ull;
-            bestTri = bestInst = 0xFFFFFFFFu;
-            bu = bv = 0.0f;
-            active = true;
-        }
-        // one step of traceInstanced's loop
-        if (ngroup.y > 0x00FFFFFFu) {
-            const uint32_t bit = 31u - __clz(ngroup.y);
-            ngroup.y &= ~(1u << bit);
-            const uint32_t slot = (bit - 24u) ^ octinv;
-            const uint32_t child = ngroup.x + __popc(ngroup.y & 0xffu & ((1u << slot) - 1u));
-            if (ngroup.y > 0x00FFFFFFu && !push(ngroup)) {
-                overflow = true;
-            }
-            uint32_t childBase, triBase, imask;
-            const uint32_t hits = intersectChildren(nodes, child, ro, idir, octinv, r.tMin, closest, childBase, triBase,
-                imask);
-            ngroup = make_uint2(childBase, (hits & 0xFF000000u) | imask);
-            tgroup = make_uint2(triBase, hits & 0x00FFFFFFu);
-        } else {
-            tgroup = ngroup;
-            ngroup = make_uint2(0u, 0u);
-        }
-        bool occluded = false;
-        while (tgroup.y != 0u) {
-            if (level == 0) {
-                // an instance: descend into its object
-                const int kt = __ffs(tgroup.y) - 1;
-                tgroup.y &= tgroup.y - 1u;
-                const uint32_t inst = __float_as_uint(__ldg(&leaves[tgroup.x + kt].v0.w));
-                bool saved = true;
-                if (ngroup.y > 0x00FFFFFFu) {
-                    saved = push(ngroup);
-                }
-                if (saved && tgroup.y != 0u) {
-                    saved = push(tgroup);
-                }
-                if (!saved) {
-                    overflow = true; // the rest of this top-level group is dropped
-                }
-                const DevInstance& I = r.S->instances[inst];
-                const DevBlas B = r.S->blases[I.meta.x];
-                curInst = inst;
-                curTriBase = B.triBase;
-                nodes = B.nodes;
-                leaves = B.tris;
-                rd = xformVector(I.w2o, r.dn);
-                setRay(xformPoint(I.w2o, r.o), rd);
-                level = 1;
-                base = sp;
-                ngroup = make_uint2(0u, B.nodeCount > 0 ? (0x80000000u | (1u << oct)) : 0u);
-                tgroup = make_uint2(0u, 0u);
-                break;
-            }
-            if (ngroup.y > 0x00FFFFFFu && __popc(__activemask()) < kPostponeLanes && push(tgroup)) {
-                break;
-            }
-            const int kt = __ffs(tgroup.y) - 1;
-            tgroup.y &= tgroup.y - 1u;
-            const TriVerts tv = leaves[tgroup.x + kt];
-            float t, u, v;
-            if (intersectTriExact(ro, rd, f3(tv.v0.x, tv.v0.y, tv.v0.z), f3(tv.v1.x, tv.v1.y, tv.v1.z),
-                    f3(tv.v2.x, tv.v2.y, tv.v2.z), r.tMin, closest, t, u, v)) {
-                const unsigned long long key = (static_cast<unsigned long long>(curInst) << 32) |
-                    static_cast<unsigned long long>(__float_as_uint(tv.v0.w));
-                if (AnyHit) {
-                    if (t < r.tMax) {
-                        occluded = true; // the first hit below tMax ends the ray
-                        break;
-                    }
-                } else if (t < closest || key > bestKey || bestKey == ~0ull) {
-                    closest = t;
-                    bestKey = key;
-                    bestTri = curTriBase + __float_as_uint(tv.v0.w);
-                    bestInst = curInst;
-                    bu = u;
-                    bv = v;
-                }
-            }
-        }
-        if (occluded) {
-            done(true);
-            continue;
-        }
-        if (ngroup.y <= 0x00FFFFFFu) {
-            if (level == 1 && sp == base) {
-                // the object is done: back to the top level in world space
-                level = 0;
-                nodes = r.S->tlasNodes;
-                leaves = r.S->tlasLeaves;
-                rd = r.dn;
-                setRay(r.o, r.dn);
-            }
-            if (sp == 0) {
-                // the ray is finished
-                done(!AnyHit && bestTri != 0xFFFFFFFFu && closest < r.tMax);
-            } else {
-                --sp;
-                ngroup = sp < kSharedStack ? sstack[sp * sstride] : stack[sp - kSharedStack];
-            }
-        }
-    }
-}
-
-// Closest hit of every queued path by the per-lane traversal.  The result of
-// queue entry k goes back into entry k (path index, bit 31 set for a miss) and
-// k_route splits the queue into the miss and hit queues in queue order
-// afterwards.  Flat scenes only (no instances, no visit counting).
-__global__ void __launch_bounds__(PT_EXTEND_LANE_THREADS, PT_EXTEND_LANE_MIN_BLOCKS)
+// Closest hit of every queued path by the whole-warp traversal.  The result of
+// queue entry k goes back into entry k (path index, bit 31 set for a miss, bit
+// 30 for a ray of quirk Q1, which k_route traces: its call would cost this
+// kernel registers) and k_route splits the queue into the miss and hit queues
+// in queue order afterwards.
+template <bool Inst, bool Multi>
+__global__ void __launch_bounds__(kTraceThreads, PT_EXTEND_LANE_MIN_BLOCKS)
     k_extend_lane(const LaunchCtx* __restrict__ cp, int sel, bool identity, int iter)
 {
     const LaunchCtx& c = *cp;
-    extern __shared__ uint2 smemStack[];
+    extern __shared__ float4 traceSmem[];
+    WarpTrace<Inst>& W = reinterpret_cast<WarpTrace<Inst>*>(traceSmem)[threadIdx.x >> 5];
     const unsigned int count = c.q.counts[sel];
     const int par = iter & 1;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -1103,70 +728,79 @@ __global__ void __launch_bounds__(PT_EXTEND_LANE_THREADS, PT_EXTEND_LANE_MIN_BLO
         c.q.counts[4 + 2 * (par ^ 1)] = 0u;
         c.q.counts[5 + 2 * (par ^ 1)] = 0u;
         c.q.counts[8 + (par ^ 1)] = 0u;
+        c.q.counts[12 + (par ^ 1)] = 0u;
     }
     uint32_t* queue = c.q.extend[sel];
-    uint32_t i = 0;
-    laneTraversal<false, PT_EXTEND_LANE_SYNC>(count, &c.q.counts[8 + par], smemStack + threadIdx.x, static_cast<int>(blockDim.x),
-        c.q.overflow,
-        [&](unsigned int k, LaneRay& r) -> bool {
+    warpTraversal<false, Inst, Multi>(c.scene, count, &c.q.counts[8 + par], W, c.q.overflow,
+        [&](unsigned int k, LaneRay& r, uint32_t& i) -> bool {
             i = identity ? k : queue[k];
-            r.S = &sceneOf(c, i);
+            r.S = Multi ? &sceneOf(c, i) : &c.scene;
             const float4 o4 = c.paths.orig[i];
             const float4 d4 = c.paths.dir[i];
             r.o = f3(o4.x, o4.y, o4.z);
             r.tMin = o4.w;
             r.tMax = kRayTMax;
             r.dn = xnormalize(f3(d4.x, d4.y, d4.z));
-            if (r.S->nodeCount != 0 && !isDegenerateDir(r.dn)) {
+            if ((Inst && r.S->instanceCount > 0) || (r.S->nodeCount != 0 && !isDegenerateDir(r.dn))) {
                 return true;
             }
-            // empty scene, or quirk Q1: decided here without the wide traversal
-            HitRec h;
-            bool hit = false;
-            h.tri = 0xFFFFFFFFu;
+            // empty scene: a miss; quirk Q1: left to k_route
             if (r.S->nodeCount != 0) {
-                hit = traceQ1(*r.S, r.o, r.dn, r.tMin, kRayTMax, false, h, c.q.overflow);
+                queue[k] = i | 0x40000000u;
+                c.q.counts[12 + par] = 1u;
+            } else {
+                queue[k] = i | 0x80000000u;
             }
-            if (hit) {
-                c.paths.hit[i] = make_float4(h.t, h.u, h.v, __uint_as_float(h.tri));
-            }
-            queue[k] = hit ? i : (i | 0x80000000u);
             return false;
         },
-        [&](unsigned int k, bool hit, float t, float u, float v, uint32_t tri) {
+        [&](unsigned int k, uint32_t i, bool hit, float t, float u, float v, uint32_t tri, uint32_t inst) {
             if (hit) {
                 c.paths.hit[i] = make_float4(t, u, v, __uint_as_float(tri));
+                if (Inst) {
+                    c.paths.hitInst[i] = inst;
+                }
             }
             queue[k] = hit ? i : (i | 0x80000000u);
         });
 }
 
-// Occlusion of every queued shadow ray by the per-lane traversal (any hit
+// Occlusion of every queued shadow ray by the whole-warp traversal (any hit
 // below the ray's tMax); unoccluded rays mark their path's pending NEE
-// contribution visible.  Flat scenes only (no instances, no visit counting).
-__global__ void __launch_bounds__(PT_EXTEND_LANE_THREADS, PT_SHADOW_LANE_MIN_BLOCKS)
+// contribution visible.
+template <bool Inst, bool Multi>
+__global__ void __launch_bounds__(kTraceThreads, PT_SHADOW_LANE_MIN_BLOCKS)
     k_shadow_lane(const LaunchCtx* __restrict__ cp, int iter)
 {
     const LaunchCtx& c = *cp;
-    extern __shared__ uint2 smemStack[];
+    extern __shared__ float4 traceSmem[];
+    WarpTrace<Inst>& W = reinterpret_cast<WarpTrace<Inst>*>(traceSmem)[threadIdx.x >> 5];
     const unsigned int count = c.q.counts[2];
     const int par = iter & 1;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         atomicAdd(&c.q.rays[1], static_cast<unsigned long long>(count));
         c.q.counts[10 + (par ^ 1)] = 0u; // next shadow stage's fetch counter
     }
-    uint32_t e = 0;
-    laneTraversal<true, PT_SHADOW_LANE_SYNC>(count, &c.q.counts[10 + par], smemStack + threadIdx.x, static_cast<int>(blockDim.x),
-        c.q.overflow,
-        [&](unsigned int k, LaneRay& r) -> bool {
+    auto visible = [&](uint32_t e) {
+        const uint32_t i = e & 0x7FFFFFFFu;
+        if (e & 0x80000000u) {
+            c.paths.visEmis[i] = 1;
+        } else {
+            c.paths.visEnv[i] = 1;
+        }
+    };
+    warpTraversal<true, Inst, Multi>(c.scene, count, &c.q.counts[10 + par], W, c.q.overflow,
+        [&](unsigned int k, LaneRay& r, uint32_t& e) -> bool {
             e = c.q.shadowPath[k];
-            r.S = &sceneOf(c, e & 0x7FFFFFFFu);
+            r.S = Multi ? &sceneOf(c, e & 0x7FFFFFFFu) : &c.scene;
             const float4 o4 = c.q.shadowOrig[k];
             const float4 d4 = c.q.shadowDir[k];
             r.o = f3(o4.x, o4.y, o4.z);
             r.dn = xnormalize(f3(d4.x, d4.y, d4.z));
             r.tMin = kShadowBias;
             r.tMax = d4.w > 0.0f ? d4.w : kRayTMax; // emitter MIS rays end short of the light
+            if (Inst && r.S->instanceCount > 0) {
+                return true;
+            }
             bool occluded = false;
             if (r.S->nodeCount != 0) {
                 if (!isDegenerateDir(r.dn)) {
@@ -1176,106 +810,29 @@ __global__ void __launch_bounds__(PT_EXTEND_LANE_THREADS, PT_SHADOW_LANE_MIN_BLO
                 occluded = traceQ1(*r.S, r.o, r.dn, r.tMin, r.tMax, true, h, c.q.overflow);
             }
             if (!occluded) {
-                const uint32_t i = e & 0x7FFFFFFFu;
-                if (e & 0x80000000u) {
-                    c.paths.visEmis[i] = 1;
-                } else {
-                    c.paths.visEnv[i] = 1;
-                }
+                visible(e);
             }
             return false;
         },
-        [&](unsigned int, bool occluded, float, float, float, uint32_t) {
+        [&](unsigned int, uint32_t e, bool occluded, float, float, float, uint32_t, uint32_t) {
             if (!occluded) {
-                const uint32_t i = e & 0x7FFFFFFFu;
-                if (e & 0x80000000u) {
-                    c.paths.visEmis[i] = 1;
-                } else {
-                    c.paths.visEnv[i] = 1;
-                }
+                visible(e);
             }
         });
 }
 
-// Closest hit of every queued path of an instanced scene by the two-level
-// per-lane traversal; results and routing as k_extend_lane.
-__global__ void __launch_bounds__(PT_EXTEND_LANE_THREADS, PT_EXTEND_LANE_MIN_BLOCKS)
-    k_extend_lane_inst(const LaunchCtx* __restrict__ cp, int sel, bool identity, int iter)
+// Closest hit of a ray with a degenerate direction (quirk Q1); its queue entry.
+static __device__ __noinline__ uint32_t routeQ1(const LaunchCtx& c, uint32_t i)
 {
-    const LaunchCtx& c = *cp;
-    extern __shared__ uint2 smemStack[];
-    const unsigned int count = c.q.counts[sel];
-    const int par = iter & 1;
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        atomicAdd(&c.q.rays[0], static_cast<unsigned long long>(count));
-        c.q.counts[sel ^ 1] = 0u;
-        c.q.counts[2] = 0u;
-        c.q.counts[3] = 0u;
-        c.q.counts[4 + 2 * (par ^ 1)] = 0u;
-        c.q.counts[5 + 2 * (par ^ 1)] = 0u;
-        c.q.counts[8 + (par ^ 1)] = 0u;
+    const DevScene& S = sceneOf(c, i);
+    const float4 o4 = c.paths.orig[i];
+    const float4 d4 = c.paths.dir[i];
+    HitRec h;
+    if (!traceQ1(S, f3(o4.x, o4.y, o4.z), xnormalize(f3(d4.x, d4.y, d4.z)), o4.w, kRayTMax, false, h, c.q.overflow)) {
+        return i | 0x80000000u;
     }
-    uint32_t* queue = c.q.extend[sel];
-    uint32_t i = 0;
-    laneTraversalInst<false>(count, &c.q.counts[8 + par], smemStack + threadIdx.x, static_cast<int>(blockDim.x),
-        c.q.overflow,
-        [&](unsigned int k, LaneRay& r) -> bool {
-            i = identity ? k : queue[k];
-            r.S = &sceneOf(c, i);
-            const float4 o4 = c.paths.orig[i];
-            const float4 d4 = c.paths.dir[i];
-            r.o = f3(o4.x, o4.y, o4.z);
-            r.tMin = o4.w;
-            r.tMax = kRayTMax;
-            r.dn = xnormalize(f3(d4.x, d4.y, d4.z));
-            return true;
-        },
-        [&](unsigned int k, bool hit, float t, float u, float v, uint32_t tri, uint32_t inst) {
-            if (hit) {
-                c.paths.hit[i] = make_float4(t, u, v, __uint_as_float(tri));
-                c.paths.hitInst[i] = inst;
-            }
-            queue[k] = hit ? i : (i | 0x80000000u);
-        });
-}
-
-// Occlusion of every queued shadow ray of an instanced scene by the two-level
-// per-lane traversal; results as k_shadow_lane.
-__global__ void __launch_bounds__(PT_EXTEND_LANE_THREADS, PT_SHADOW_LANE_MIN_BLOCKS)
-    k_shadow_lane_inst(const LaunchCtx* __restrict__ cp, int iter)
-{
-    const LaunchCtx& c = *cp;
-    extern __shared__ uint2 smemStack[];
-    const unsigned int count = c.q.counts[2];
-    const int par = iter & 1;
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        atomicAdd(&c.q.rays[1], static_cast<unsigned long long>(count));
-        c.q.counts[10 + (par ^ 1)] = 0u; // next shadow stage's fetch counter
-    }
-    uint32_t e = 0;
-    laneTraversalInst<true>(count, &c.q.counts[10 + par], smemStack + threadIdx.x, static_cast<int>(blockDim.x),
-        c.q.overflow,
-        [&](unsigned int k, LaneRay& r) -> bool {
-            e = c.q.shadowPath[k];
-            r.S = &sceneOf(c, e & 0x7FFFFFFFu);
-            const float4 o4 = c.q.shadowOrig[k];
-            const float4 d4 = c.q.shadowDir[k];
-            r.o = f3(o4.x, o4.y, o4.z);
-            r.dn = xnormalize(f3(d4.x, d4.y, d4.z));
-            r.tMin = kShadowBias;
-            r.tMax = d4.w > 0.0f ? d4.w : kRayTMax; // emitter MIS rays end short of the light
-            return true;
-        },
-        [&](unsigned int, bool occluded, float, float, float, uint32_t, uint32_t) {
-            if (!occluded) {
-                const uint32_t i = e & 0x7FFFFFFFu;
-                if (e & 0x80000000u) {
-                    c.paths.visEmis[i] = 1;
-                } else {
-                    c.paths.visEnv[i] = 1;
-                }
-            }
-        });
+    c.paths.hit[i] = make_float4(h.t, h.u, h.v, __uint_as_float(h.tri));
+    return i;
 }
 
 // Splits the queue that k_extend_lane marked into the miss and hit queues of
@@ -1291,13 +848,21 @@ __global__ void __launch_bounds__(256) k_route(const LaunchCtx* __restrict__ cp,
     const LaunchCtx& c = *cp;
     const unsigned int count = c.q.counts[sel];
     const int par = iter & 1;
-    const uint32_t* queue = c.q.extend[sel];
+    uint32_t* queue = c.q.extend[sel];
+    const bool q1 = c.q.counts[12 + par] != 0u;
     __shared__ unsigned int sHit[kRouteRows * 8], sMiss[kRouteRows * 8]; // exclusive offsets per (row, warp)
     __shared__ unsigned int sBase[2];
     const unsigned int lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const unsigned int below = (1u << lane) - 1u;
     const unsigned int tile = 256u * kRouteRows;
     for (unsigned int t0 = blockIdx.x * tile; t0 < count; t0 += gridDim.x * tile) {
+        if (q1) {
+            for (unsigned int k = t0 + threadIdx.x; k < min(t0 + tile, count); k += 256u) {
+                if ((queue[k] & 0x40000000u) != 0u) {
+                    queue[k] = routeQ1(c, queue[k] & 0x3FFFFFFFu);
+                }
+            }
+        }
         uint32_t e[kRouteRows];
         unsigned int hitMask[kRouteRows], missMask[kRouteRows];
 #pragma unroll
@@ -2111,26 +1676,39 @@ void launchGenerate(const LaunchCtx* d, int count, int extendSel, int nw, cudaSt
         k_generate<0><<<gridFor(count), 256, 0, s>>>(d, count, extendSel, jobOffset);
     }
 }
+namespace {
+template <bool Inst> constexpr size_t traceSmemBytes() { return sizeof(WarpTrace<Inst>) * (kTraceThreads / 32); }
+static_assert(traceSmemBytes<true>() <= 48 * 1024, "dynamic shared memory without opting in");
+template <class F> int blocksPerSm(F kernel, int threads, size_t smem)
+{
+    int blocks = 1;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, kernel, threads, smem);
+    return blocks > 0 ? blocks : 1;
+}
+} // namespace
 void launchExtend(const LaunchCtx* c, int sel, bool identity, int iter, int grid, bool count, bool inst, bool lane,
-    cudaStream_t s)
+    bool multi, cudaStream_t s)
 {
     const size_t smem = sizeof(uint2) * kSharedStack * 256;
-    if (inst) {
+    if (lane && !count) {
+        if (inst && multi) {
+            k_extend_lane<true, true><<<grid, kTraceThreads, traceSmemBytes<true>(), s>>>(c, sel, identity, iter);
+        } else if (inst) {
+            k_extend_lane<true, false><<<grid, kTraceThreads, traceSmemBytes<true>(), s>>>(c, sel, identity, iter);
+        } else if (multi) {
+            k_extend_lane<false, true><<<grid, kTraceThreads, traceSmemBytes<false>(), s>>>(c, sel, identity, iter);
+        } else {
+            k_extend_lane<false, false><<<grid, kTraceThreads, traceSmemBytes<false>(), s>>>(c, sel, identity, iter);
+        }
+        k_route<<<grid, 256, 0, s>>>(c, sel, iter);
+    } else if (inst) {
         if (count) {
             k_extend<true, true><<<grid, 256, smem, s>>>(c, sel, identity, iter);
-        } else if (lane) {
-            k_extend_lane_inst<<<grid, PT_EXTEND_LANE_THREADS, sizeof(uint2) * kSharedStack * PT_EXTEND_LANE_THREADS,
-                s>>>(c, sel, identity, iter);
-            k_route<<<grid, 256, 0, s>>>(c, sel, iter);
         } else {
             k_extend<false, true><<<grid, 256, smem, s>>>(c, sel, identity, iter);
         }
     } else if (count) {
         k_extend<true, false><<<grid, 256, smem, s>>>(c, sel, identity, iter);
-    } else if (lane) {
-        k_extend_lane<<<grid, PT_EXTEND_LANE_THREADS, sizeof(uint2) * kSharedStack * PT_EXTEND_LANE_THREADS, s>>>(c, sel,
-            identity, iter);
-        k_route<<<grid, 256, 0, s>>>(c, sel, iter);
     } else {
         k_extend<false, false><<<grid, 256, smem, s>>>(c, sel, identity, iter);
     }
@@ -2143,38 +1721,26 @@ void launchNextQueue(const LaunchCtx* c, int sel, int grid, cudaStream_t s)
 {
     k_next_queue<<<grid, 256, 0, s>>>(c, sel);
 }
+int extendLaneOccupancy()
+{
+    return blocksPerSm(k_extend_lane<false, false>, kTraceThreads, traceSmemBytes<false>());
+}
 int extendLaneInstOccupancy()
 {
-    int blocks = 1;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k_extend_lane_inst, PT_EXTEND_LANE_THREADS,
-        sizeof(uint2) * kSharedStack * PT_EXTEND_LANE_THREADS);
-    return blocks > 0 ? blocks : 1;
-}
-int shadowLaneInstOccupancy()
-{
-    int blocks = 1;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k_shadow_lane_inst, PT_EXTEND_LANE_THREADS,
-        sizeof(uint2) * kSharedStack * PT_EXTEND_LANE_THREADS);
-    return blocks > 0 ? blocks : 1;
+    return blocksPerSm(k_extend_lane<true, false>, kTraceThreads, traceSmemBytes<true>());
 }
 int shadowLaneOccupancy()
 {
-    int blocks = 1;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k_shadow_lane, PT_EXTEND_LANE_THREADS,
-        sizeof(uint2) * kSharedStack * PT_EXTEND_LANE_THREADS);
-    return blocks > 0 ? blocks : 1;
+    return blocksPerSm(k_shadow_lane<false, false>, kTraceThreads, traceSmemBytes<false>());
+}
+int shadowLaneInstOccupancy()
+{
+    return blocksPerSm(k_shadow_lane<true, false>, kTraceThreads, traceSmemBytes<true>());
 }
 int shadeMissOccupancy()
 {
     int blocks = 1;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k_shade_miss<8>, 256, 0);
-    return blocks > 0 ? blocks : 1;
-}
-int extendLaneOccupancy()
-{
-    int blocks = 1;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k_extend_lane, PT_EXTEND_LANE_THREADS,
-        sizeof(uint2) * kSharedStack * PT_EXTEND_LANE_THREADS);
     return blocks > 0 ? blocks : 1;
 }
 void launchShadeMiss(const LaunchCtx* c, int iter, int sel, int grid, int nw, cudaStream_t s)
@@ -2197,16 +1763,18 @@ void launchShade(const LaunchCtx* c, int sel, int iter, int grid, int nw, cudaSt
         k_shade<0><<<grid, 256, 0, s>>>(c, sel, iter);
     }
 }
-void launchShadow(const LaunchCtx* c, int iter, int grid, bool count, bool inst, bool lane, cudaStream_t s)
+void launchShadow(const LaunchCtx* c, int iter, int grid, bool count, bool inst, bool lane, bool multi, cudaStream_t s)
 {
     const size_t smem = sizeof(uint2) * kSharedStack * 256;
-    if (PT_SHADOW_LANE && lane && !count) {
-        if (inst) {
-            k_shadow_lane_inst<<<grid, PT_EXTEND_LANE_THREADS, sizeof(uint2) * kSharedStack * PT_EXTEND_LANE_THREADS,
-                s>>>(c, iter);
+    if (lane && !count) {
+        if (inst && multi) {
+            k_shadow_lane<true, true><<<grid, kTraceThreads, traceSmemBytes<true>(), s>>>(c, iter);
+        } else if (inst) {
+            k_shadow_lane<true, false><<<grid, kTraceThreads, traceSmemBytes<true>(), s>>>(c, iter);
+        } else if (multi) {
+            k_shadow_lane<false, true><<<grid, kTraceThreads, traceSmemBytes<false>(), s>>>(c, iter);
         } else {
-            k_shadow_lane<<<grid, PT_EXTEND_LANE_THREADS, sizeof(uint2) * kSharedStack * PT_EXTEND_LANE_THREADS, s>>>(c,
-                iter);
+            k_shadow_lane<false, false><<<grid, kTraceThreads, traceSmemBytes<false>(), s>>>(c, iter);
         }
     } else if (inst) {
         if (count) {

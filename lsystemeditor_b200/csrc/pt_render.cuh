@@ -68,7 +68,8 @@ struct QueueSet {
     float4* shadowDir = nullptr;
     // counters: [0],[1] extend ping-pong, [2] shadow, [3] finish,
     // [4 + 2p] misses / [5 + 2p] hits of bounce parity p, [8 + p] extend and
-    // [10 + p] shadow work-fetch counters
+    // [10 + p] shadow work-fetch counters, [12 + p] nonzero: k_extend_lane left
+    // rays of quirk Q1 to k_route
     unsigned int* counts = nullptr;
     unsigned long long* rays = nullptr;       // [0] closest-hit rays, [1] shadow rays
     unsigned long long* visits = nullptr;     // [0..1] extend nodes/tris, [2..3] shadow nodes/tris
@@ -166,7 +167,7 @@ void launchGenerate(const LaunchCtx* d, int count, int extendSel, int nw, cudaSt
 // Closest-hit stage.  lane: per-lane ray replacement (k_extend_lane + k_route;
 // flat scenes, no visit counting), else one warp-fetch k_extend.
 void launchExtend(const LaunchCtx* d, int sel, bool identity, int iter, int grid, bool count, bool inst, bool lane,
-    cudaStream_t s);
+    bool multi, cudaStream_t s);
 // Kernels one launchExtend call launches (closest hit, and the routing pass after it).
 int extendKernels(bool count, bool inst, bool lane);
 // Resident blocks per SM of the per-lane closest-hit kernel and of the miss shader.
@@ -183,7 +184,7 @@ void launchShadeMiss(const LaunchCtx* d, int iter, int sel, int grid, int nw, cu
 void launchShade(const LaunchCtx* d, int sel, int iter, int grid, int nw, cudaStream_t s);
 // Shadow stage.  lane: per-lane ray replacement (k_shadow_lane; flat scenes,
 // no visit counting), else one warp per 32 queued rays (k_shadow).
-void launchShadow(const LaunchCtx* d, int iter, int grid, bool count, bool inst, bool lane, cudaStream_t s);
+void launchShadow(const LaunchCtx* d, int iter, int grid, bool count, bool inst, bool lane, bool multi, cudaStream_t s);
 void launchFinalize(const LaunchCtx* d, int sel, int grid, int nw, cudaStream_t s);
 void launchAccumulate(const LaunchCtx* d, int activeCount, int batch, cudaStream_t s);
 // Stable compaction of the active list (pixels neither converged nor at the

@@ -1,0 +1,409 @@
+// Traversal of a queue of rays by whole warps (closest hit or any hit; flat
+// scenes, or the two-level BVH of instanced ones).
+//
+// Every lane owns one ray; the warp steps together:
+//   fetch   when at least kFetchLanes lanes are idle they take the next
+//           entries of the warp's chunk of the queue (one atomic per chunk);
+//   node    every lane that has no triangles to test intersects the eight
+//           children of its next node;
+//   round   the (ray, triangle) pairs that the lanes hold are dealt out to
+//           the lanes, 32 at a time: a lane tests whichever pair it gets, with
+//           the owner's ray from shared memory, and the closest hit of each
+//           owner is settled by a 64-bit minimum over (t, ~triangle id).  A
+//           round runs when the pairs fill at least kRoundPairs lanes, or no
+//           lane can do a node step.  Lanes with pairs left wait, so a ray
+//           tests a node's triangles before its next node, as traceRay does.
+//   pop     lanes without work take the next group from their stack, or finish;
+//   steal   (flat scenes) once the queue is drained, idle lanes take the oldest
+//           stack entry of busy lanes and traverse that part of their ray, so
+//           that a launch does not wait for one lane's long ray.
+//
+// Why: in a free-running loop (a lane fetched and stepped on its own) 6 of 32
+// lanes worked per executed instruction, a node's triangles were tested one
+// after the other, and every finished ray was an atomic on one address.  It is
+// bound by the latency of the node and triangle loads and by issue (16 of 32
+// lanes, 45% of the issue slots; DRAM idles, the scene is in L2).  Registers
+// matter more than warps: with spills at 64 registers it lost a quarter, so the
+// per-ray words that only the ends of a ray need are in shared memory, and
+// rays of quirk Q1 are traced elsewhere (their call costs registers here).
+// Measured: closest hit of the large frame (972k triangles, 402M rays) 159.9 ->
+// 85.4 ms, of one 1024^2 wave (1.6M rays over 8 launches) 1.86 -> 0.95 ms (1.34
+// without stealing: the launches of late bounces wait for their longest ray),
+// shadow rays of a 513x511 32-spp emitter-MIS frame 3.73 -> 2.10 ms.
+#pragma once
+
+#include "pt_trace.cuh"
+
+#include <type_traits>
+
+namespace pt {
+
+#ifndef PT_TRACE_STACK
+#define PT_TRACE_STACK 16
+#endif
+#ifndef PT_FETCH_LANES
+#define PT_FETCH_LANES 8
+#endif
+#ifndef PT_ROUND_PAIRS
+#define PT_ROUND_PAIRS 20
+#endif
+#ifndef PT_TRACE_CHUNK
+#define PT_TRACE_CHUNK 128
+#endif
+constexpr int kTraceThreads = 128;
+constexpr int kTraceStack = PT_TRACE_STACK;       // stack entries per lane in shared memory (the rest is local)
+constexpr int kFetchLanes = PT_FETCH_LANES;
+constexpr int kRoundPairs = PT_ROUND_PAIRS;
+constexpr unsigned int kTraceChunk = PT_TRACE_CHUNK;
+
+// A ray: its scene, origin, normalised direction and the parametric interval it is tested on.
+struct LaneRay {
+    const DevScene* S;
+    float3 o;
+    float3 dn;
+    float tMin;
+    float tMax;
+};
+
+struct TraceInstPart {
+    float4 wo[32];    // world ray (o / d below are the object's while inside one)
+    float4 wd[32];
+    uint2 cur[32];    // instance being traversed, first shading record of its object
+};
+struct TraceNoInst {};
+
+// A warp's shared memory.
+template <bool Inst> struct WarpTrace {
+    float4 o[32];                 // ray origin, tMin
+    float4 d[32];                 // ray direction
+    float4 res[32];               // u, v, triangle, instance of the best hit so far
+    uint2 entry[32];              // queue entry, caller's word
+    unsigned int lanes[32];       // lanes that traverse this ray
+    unsigned long long key[32];   // closest t << 32 | ~(id of that hit); see warpTraversal
+    uint2 stack[kTraceStack][32];
+    uint2 give[32];               // stack entries handed to idle lanes
+    uint16_t pair[32];            // owner lane | its ray << 5 | triangle bit << 10
+    std::conditional_t<Inst, TraceInstPart, TraceNoInst> in;
+};
+
+//   load(k, ray, word) -> bool: reads queue entry k (word: kept for finish);
+//     false when the entry was decided without the wide traversal.
+//   finish(k, word, hit, t, u, v, tri, inst): the result of entry k (for AnyHit,
+//     hit means occluded and the rest is unset).
+// Multi: rays of several scenes (their node and triangle arrays differ per lane).
+// Ties: of several hits at exactly the same t the highest original triangle id
+// wins (instanced: the highest (instance, triangle)), as in traceRay.
+template <bool AnyHit, bool Inst, bool Multi, class Load, class Finish>
+__device__ __forceinline__ void warpTraversal(const DevScene& S0, unsigned int count, unsigned int* fetch,
+    WarpTrace<Inst>& W, unsigned int* overflowCounter, Load load, Finish finish)
+{
+    constexpr unsigned int kAll = 0xFFFFFFFFu;
+    constexpr bool kPerRay = Inst || Multi;
+    const unsigned int lane = threadIdx.x & 31u;
+    const unsigned int below = (1u << lane) - 1u;
+    uint2 spill[kTraversalStack];
+    bool active = false, overflow = false;
+    unsigned int ray = lane; // the ray (index into W) that this lane traverses
+    float3 o = f3(0.0f, 0.0f, 0.0f), idir = o;
+    float tMin = 0.0f, closest = 0.0f;
+    uint32_t octinv = 0;
+    uint2 ngroup = make_uint2(0u, 0u), tgroup = make_uint2(0u, 0u);
+    int sp = 0, sb = 0; // stack entries sb .. sp - 1
+    const DevScene* S = &S0;
+    const CwNode* nodes = Inst ? nullptr : S0.nodes;
+    const TriVerts* tris = Inst ? nullptr : S0.tris;
+    int level = 0, base = 0;
+    // the warp's chunk of the queue; small queues are spread over all warps
+    unsigned int poolNext = 0, poolEnd = 0;
+    bool drained = false;
+    const unsigned int warps = gridDim.x * (kTraceThreads / 32);
+    const unsigned int chunk = min(kTraceChunk, max(1u, count / (warps * 2u)));
+
+    auto push = [&](uint2 g) -> bool {
+        if (sp < kTraceStack) {
+            W.stack[sp][lane] = g;
+        } else if (sp < kTraceStack + kTraversalStack) {
+            spill[sp - kTraceStack] = g;
+        } else {
+            return false;
+        }
+        ++sp;
+        return true;
+    };
+    auto setRay = [&](float3 a, float3 d) {
+        o = a;
+        if constexpr (Inst) {
+            d.x = fabsf(d.x) < 1.0e-20f ? copysignf(1.0e-20f, d.x) : d.x;
+            d.y = fabsf(d.y) < 1.0e-20f ? copysignf(1.0e-20f, d.y) : d.y;
+            d.z = fabsf(d.z) < 1.0e-20f ? copysignf(1.0e-20f, d.z) : d.z;
+        }
+        idir = f3(__frcp_rn(d.x), __frcp_rn(d.y), __frcp_rn(d.z));
+        octinv = 7u - ((d.x < 0.0f ? 4u : 0u) | (d.y < 0.0f ? 2u : 0u) | (d.z < 0.0f ? 1u : 0u));
+    };
+    // every slot's octant of the root group: only slot 0 exists
+    auto rootGroup = [&]() { return make_uint2(0u, 0x80000000u | (1u << (7u - octinv))); };
+    for (;;) {
+        const unsigned int idle = __ballot_sync(kAll, !active);
+        if (!drained && __popc(idle) >= kFetchLanes) {
+            if (poolNext >= poolEnd) {
+                unsigned int b = 0;
+                if (lane == 0) {
+                    b = atomicAdd(fetch, chunk);
+                }
+                poolNext = __shfl_sync(kAll, b, 0);
+                poolEnd = min(poolNext + chunk, count);
+                drained = poolNext >= count;
+            }
+            if (!drained) {
+                const unsigned int n = min(static_cast<unsigned int>(__popc(idle)), poolEnd - poolNext);
+                const unsigned int r = __popc(idle & below);
+                if (!active && r < n) {
+                    const unsigned int k = poolNext + r;
+                    LaneRay q;
+                    uint32_t word = 0;
+                    if (load(k, q, word)) {
+                        W.entry[lane] = make_uint2(k, word);
+                        W.lanes[lane] = 1u;
+                        W.o[lane] = make_float4(q.o.x, q.o.y, q.o.z, q.tMin);
+                        W.d[lane] = make_float4(q.dn.x, q.dn.y, q.dn.z, 0.0f);
+                        if constexpr (Inst) {
+                            W.in.wo[lane] = make_float4(q.o.x, q.o.y, q.o.z, 0.0f);
+                            W.in.wd[lane] = make_float4(q.dn.x, q.dn.y, q.dn.z, 0.0f);
+                        }
+                        // (low word 0: a hit at exactly tMax does not count)
+                        W.key[lane] = static_cast<unsigned long long>(__float_as_uint(q.tMax)) << 32;
+                        W.res[lane] = make_float4(0.0f, 0.0f, __uint_as_float(0xFFFFFFFFu), __uint_as_float(0xFFFFFFFFu));
+                        setRay(q.o, q.dn);
+                        tMin = q.tMin;
+                        closest = q.tMax;
+                        if constexpr (kPerRay) {
+                            S = q.S;
+                            // (a flat scene of an instanced batch starts inside its only object)
+                            const bool flat = !Inst || S->instanceCount == 0;
+                            nodes = flat ? S->nodes : S->tlasNodes;
+                            tris = flat ? S->tris : S->tlasLeaves;
+                            if constexpr (Inst) {
+                                W.in.cur[lane] = make_uint2(0xFFFFFFFFu, 0u);
+                                level = flat ? 1 : 0;
+                                base = 0;
+                            }
+                        }
+                        sp = sb = 0;
+                        ngroup = rootGroup();
+                        tgroup = make_uint2(0u, 0u);
+                        active = true;
+                    }
+                }
+                poolNext += n;
+            }
+        }
+        if (drained) {
+            if (idle == kAll) {
+                break;
+            }
+            if constexpr (!Inst) {
+                const bool gives = active && sp > sb && sb < kTraceStack;
+                const unsigned int victims = __ballot_sync(kAll, gives);
+                if (idle != 0u && victims != 0u) {
+                    const unsigned int n = min(__popc(idle), __popc(victims));
+                    const unsigned int r = __popc((active ? victims : idle) & below);
+                    if (gives && r < n) {
+                        W.pair[r] = static_cast<uint16_t>(lane | (ray << 5));
+                        W.give[r] = W.stack[sb][lane];
+                        ++sb;
+                        atomicAdd(&W.lanes[ray], 1u);
+                    }
+                    __syncwarp();
+                    const bool takes = !active && r < n;
+                    const unsigned int p = takes ? W.pair[r] : lane;
+                    if constexpr (Multi) {
+                        const unsigned long long np = __shfl_sync(kAll, reinterpret_cast<unsigned long long>(nodes), p & 31u);
+                        const unsigned long long tp = __shfl_sync(kAll, reinterpret_cast<unsigned long long>(tris), p & 31u);
+                        if (takes) {
+                            nodes = reinterpret_cast<const CwNode*>(np);
+                            tris = reinterpret_cast<const TriVerts*>(tp);
+                        }
+                    }
+                    if (takes) {
+                        ray = p >> 5;
+                        const float4 ro = W.o[ray], rd = W.d[ray];
+                        setRay(f3(ro.x, ro.y, ro.z), f3(rd.x, rd.y, rd.z));
+                        tMin = ro.w;
+                        closest = __uint_as_float(static_cast<uint32_t>(W.key[ray] >> 32));
+                        ngroup = W.give[r];
+                        tgroup = make_uint2(0u, 0u);
+                        sp = sb = 0;
+                        active = true;
+                    }
+                    __syncwarp(); // the pair list is rewritten by the triangle round
+                }
+            }
+        }
+        // --- node step (lanes whose triangles are all tested) ---
+        if (active && tgroup.y == 0u && (!Inst || ngroup.y > 0x00FFFFFFu)) {
+            const uint32_t bit = 31u - __clz(ngroup.y);
+            ngroup.y &= ~(1u << bit);
+            const uint32_t slot = (bit - 24u) ^ octinv;
+            const uint32_t child = ngroup.x + __popc(ngroup.y & 0xffu & ((1u << slot) - 1u));
+            if (ngroup.y > 0x00FFFFFFu && !push(ngroup)) {
+                overflow = true;
+            }
+            uint32_t childBase, triBase, imask;
+            const uint32_t hits = intersectChildren(nodes, child, o, idir, octinv, tMin, closest, childBase, triBase, imask);
+            ngroup = make_uint2(childBase, (hits & 0xFF000000u) | imask);
+            tgroup = make_uint2(triBase, hits & 0x00FFFFFFu);
+        }
+        if constexpr (Inst) {
+            if (level == 0 && tgroup.y != 0u) {
+                // an instance: descend into its object
+                const int kt = __ffs(tgroup.y) - 1;
+                tgroup.y &= tgroup.y - 1u;
+                const uint32_t inst = __float_as_uint(__ldg(&tris[tgroup.x + kt].v0.w));
+                bool saved = true;
+                if (ngroup.y > 0x00FFFFFFu) {
+                    saved = push(ngroup);
+                }
+                if (saved && tgroup.y != 0u) {
+                    saved = push(tgroup);
+                }
+                if (!saved) {
+                    overflow = true; // the rest of this top-level group is dropped
+                }
+                const DevInstance& I = S->instances[inst];
+                const DevBlas B = S->blases[I.meta.x];
+                nodes = B.nodes;
+                tris = B.tris;
+                const float4 wo = W.in.wo[lane], wd = W.in.wd[lane];
+                const float3 od = xformVector(I.w2o, f3(wd.x, wd.y, wd.z));
+                setRay(xformPoint(I.w2o, f3(wo.x, wo.y, wo.z)), od);
+                W.o[lane] = make_float4(o.x, o.y, o.z, tMin);
+                W.d[lane] = make_float4(od.x, od.y, od.z, 0.0f);
+                W.in.cur[lane] = make_uint2(inst, B.triBase);
+                if constexpr (!AnyHit) {
+                    // at an exact tie this instance's triangles win or lose as a whole
+                    // (an instance is a single top-level leaf)
+                    const uint32_t bi = __float_as_uint(W.res[lane].w);
+                    const bool wins = bi != 0xFFFFFFFFu && inst > bi;
+                    W.key[lane] = (static_cast<unsigned long long>(__float_as_uint(closest)) << 32) | (wins ? 0xFFFFFFFFull : 0ull);
+                }
+                level = 1;
+                base = sp;
+                ngroup = B.nodeCount > 0 ? rootGroup() : make_uint2(0u, 0u);
+                tgroup = make_uint2(0u, 0u);
+            }
+        }
+        // --- triangle round ---
+        {
+            const unsigned int c = min(__popc(tgroup.y), 7);
+            const unsigned int b0 = __ballot_sync(kAll, (c & 1u) != 0u);
+            const unsigned int b1 = __ballot_sync(kAll, (c & 2u) != 0u);
+            const unsigned int b2 = __ballot_sync(kAll, (c & 4u) != 0u);
+            const int total = __popc(b0) + 2 * __popc(b1) + 4 * __popc(b2);
+            const bool canStep = active && tgroup.y == 0u;
+            if (total >= kRoundPairs || (total > 0 && !__any_sync(kAll, canStep))) {
+                const unsigned int off = __popc(b0 & below) + 2 * __popc(b1 & below) + 4 * __popc(b2 & below);
+                const unsigned int end = min(off + c, 32u);
+                for (unsigned int j = off; j < end; ++j) {
+                    const unsigned int kt = __ffs(tgroup.y) - 1;
+                    tgroup.y &= tgroup.y - 1u;
+                    W.pair[j] = static_cast<uint16_t>(lane | (ray << 5) | (kt << 10));
+                }
+                __syncwarp();
+                const bool mine = static_cast<int>(lane) < total;
+                const unsigned int p = mine ? W.pair[lane] : lane;
+                const unsigned int owner = p & 31u, oray = (p >> 5) & 31u;
+                const uint32_t tb = __shfl_sync(kAll, tgroup.x, owner);
+                const TriVerts* tp = tris;
+                if constexpr (kPerRay) {
+                    tp = reinterpret_cast<const TriVerts*>(
+                        __shfl_sync(kAll, reinterpret_cast<unsigned long long>(tris), owner));
+                }
+                bool hit = false;
+                float t = 0.0f, u = 0.0f, v = 0.0f;
+                uint32_t id = 0;
+                unsigned long long nk = 0;
+                if (mine) {
+                    const TriVerts tv = tp[tb + (p >> 10)];
+                    const float4 ro = W.o[oray], rd = W.d[oray];
+                    const float cl = __uint_as_float(static_cast<uint32_t>(W.key[oray] >> 32));
+                    hit = intersectTriExact(f3(ro.x, ro.y, ro.z), f3(rd.x, rd.y, rd.z), f3(tv.v0.x, tv.v0.y, tv.v0.z),
+                        f3(tv.v1.x, tv.v1.y, tv.v1.z), f3(tv.v2.x, tv.v2.y, tv.v2.z), ro.w, cl, t, u, v);
+                    if constexpr (AnyHit) {
+                        hit = hit && t < cl;
+                    } else if (hit) {
+                        id = __float_as_uint(tv.v0.w);
+                        // (t >= tMin >= 0: the bits order like the values; -0 counts as 0)
+                        nk = (static_cast<unsigned long long>(__float_as_uint(__fadd_rn(t, 0.0f))) << 32) | (~id);
+                    }
+                }
+                if (__any_sync(kAll, hit)) {
+                    if constexpr (AnyHit) {
+                        if (hit) {
+                            W.res[oray].x = 1.0f;
+                        }
+                        __syncwarp();
+                        if (active && W.res[ray].x != 0.0f) {
+                            tgroup.y = 0u; // occluded: the ray ends below
+                            ngroup.y = 0u;
+                            sp = sb;
+                        }
+                    } else {
+                        if (hit) {
+                            atomicMin(&W.key[oray], nk);
+                        }
+                        __syncwarp();
+                        if (hit && W.key[oray] == nk) {
+                            if constexpr (Inst) {
+                                const uint2 cur = W.in.cur[oray];
+                                W.res[oray] = make_float4(u, v, __uint_as_float(cur.y + id), __uint_as_float(cur.x));
+                            } else {
+                                W.res[oray] = make_float4(u, v, __uint_as_float(id), 0.0f);
+                            }
+                        }
+                        if (active) {
+                            closest = __uint_as_float(static_cast<uint32_t>(W.key[ray] >> 32));
+                        }
+                    }
+                }
+                __syncwarp(); // the pair list, keys and rays are rewritten after this
+            }
+        }
+        // --- pop ---
+        if (active && tgroup.y == 0u && ngroup.y <= 0x00FFFFFFu) {
+            if constexpr (Inst) {
+                if (level == 1 && sp == base && sp > 0) { // (sb is 0: no stealing)
+                    // the object is done: back to the top level in world space
+                    level = 0;
+                    nodes = S->tlasNodes;
+                    tris = S->tlasLeaves;
+                    const float4 wo = W.in.wo[lane], wd = W.in.wd[lane];
+                    setRay(f3(wo.x, wo.y, wo.z), f3(wd.x, wd.y, wd.z));
+                }
+            }
+            if (sp == sb) {
+                // (the last lane of a ray finishes it)
+                if (Inst || atomicSub(&W.lanes[ray], 1u) == 1u) {
+                    const float4 rs = W.res[ray];
+                    const uint2 en = W.entry[ray];
+                    const bool h = AnyHit ? rs.x != 0.0f : __float_as_uint(rs.z) != 0xFFFFFFFFu;
+                    finish(en.x, en.y, h, closest, rs.x, rs.y, __float_as_uint(rs.z), __float_as_uint(rs.w));
+                }
+                if (overflow && overflowCounter != nullptr && !(AnyHit && W.res[ray].x != 0.0f)) {
+                    atomicAdd(overflowCounter, 1u); // rays whose stack overflowed (an occluded any-hit ray is not counted)
+                }
+                overflow = false;
+                active = false;
+            } else {
+                --sp;
+                const uint2 g = sp < kTraceStack ? W.stack[sp][lane] : spill[sp - kTraceStack];
+                if (!Inst || g.y > 0x00FFFFFFu) {
+                    ngroup = g;
+                } else {
+                    tgroup = g; // the rest of a top-level leaf group
+                }
+            }
+        }
+    }
+}
+
+} // namespace pt
