@@ -1,8 +1,7 @@
 """Whole-warp traversal (csrc/pt_traverse.cuh) and the plane decode of the
 compressed nodes (csrc/pt_trace.cuh).
 
-* CPU: the decoded near / far plane parameters bracket the exact ones for
-  node scales, directions and origins over the ranges that a scene can have.
+* CPU: the permute-and-subtract decode gives every plane byte exactly.
 * GPU: the whole-warp kernels render what the one-ray-per-lane traversal
   renders, bit for bit, where their bookkeeping has edges: fewer rays than
   lanes, one more than a warp, a chunk or a block, single-triangle scenes, every
@@ -17,31 +16,22 @@ from lsystemeditor_b200.scene import HostMesh, placement
 from tests.helpers import random_soup, zoo_camera, zoo_scene
 
 
-def test_plane_decode_is_conservative():
-    rng = np.random.default_rng(7)
-    n = 400_000
+def test_plane_decode_is_exact():
+    """Byte j of a plane word placed under 0x4B0000.. (2^23) and 2^23 subtracted is float(byte): the plane
+    parameters are then those of fmaf(float(q), a, b), whatever a and b."""
     f = np.float32
-    scale = np.ldexp(f(1.0), rng.integers(-30, 8, n)).astype(f)
-    idir = (np.exp(rng.normal(0.0, 4.0, n)) * rng.choice([-1.0, 1.0], n)).astype(f)
-    q = rng.integers(0, 256, n)
-    # origins from inside the node to 2^20 of its extents away
-    p = rng.normal(0.0, 5.0, n).astype(f)
-    o = (p + scale * 256.0 * rng.uniform(-1.0, 1.0, n) * np.exp2(rng.uniform(-4.0, 20.0, n))).astype(f)
-    rel = (p - o).astype(f)
-    exact = (q * scale.astype(np.float64) + rel) * idir          # the plane's parameter from the rounded p - o
-    a = (scale * f(32768.0) * idir).astype(f)
-    b = (rel.astype(np.float64) * idir - a).astype(f)            # fma: one rounding
-    pad = np.abs(a).astype(np.float64) * 2.0 ** -22
-    near, far = (b - pad).astype(f), (b + pad).astype(f)
-    plane = (f(1.0) + q.astype(f) * f(2.0 ** -15)).astype(f)
-    assert np.array_equal((plane.view(np.uint32) >> 8) & 0xFF, q), "the byte sits in bits 8..15"
-    t0 = (plane.astype(np.float64) * a + near).astype(f)
-    t1 = (plane.astype(np.float64) * a + far).astype(f)
-    slack = np.abs(exact) * 2.0 ** -22                           # half of what the slab test's tExit is widened by
-    assert np.all(t0 <= exact + slack) and np.all(t1 >= exact - slack)
-    # and the boxes stay tight: within 1/64 of a quantum (plus rounding)
-    quantum = np.abs(scale.astype(np.float64) * idir)
-    assert np.all(t1.astype(np.float64) - t0 <= quantum / 32.0 + np.abs(exact) * 2.0 ** -21)
+    words = (np.arange(256, dtype=np.uint64)[:, None] * np.array([1, 1 << 8, 1 << 16, 1 << 24], np.uint64)).astype(np.uint32)
+    words = words | np.uint32(0x5A5A5A5A) & ~np.array([0xFF, 0xFF00, 0xFF0000, 0xFF000000], np.uint32)
+    for j in range(4):
+        sources = np.concatenate([words[:, j].copy().view(np.uint8).reshape(-1, 4),
+                                  np.broadcast_to(np.array([0, 0, 0, 0x4B], np.uint8), (256, 4))], 1)
+        for first in (0x7540, 0x7541):  # the two lanes of a pair; the kernel adds the pair's first byte
+            if (first & 1) != (j & 1):
+                continue
+            selector = first + (j & 2)
+            picked = sources[:, [(selector >> (4 * k)) & 7 for k in range(4)]]
+            q = np.ascontiguousarray(picked).view(np.uint32).reshape(-1).view(f) - f(8388608.0)
+            assert np.array_equal(q, np.arange(256, dtype=f))
 
 
 def _images(t, mode):
