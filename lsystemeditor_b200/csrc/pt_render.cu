@@ -343,6 +343,21 @@ template <int NW> __device__ __forceinline__ Col<NW> skyCol(const LaunchCtx& c, 
     return L;
 }
 
+// No light comes from the sky at all: a black background, no distant light.
+template <int NW> __device__ __forceinline__ bool skyIsBlack(const LaunchCtx& c)
+{
+    if (c.sun.enabled != 0 || c.env.valid) {
+        return false;
+    }
+    if constexpr (NW == 0) {
+        const float k = c.params.environment_intensity;
+        return c.params.background_r * k == 0.0f && c.params.background_g * k == 0.0f && c.params.background_b * k == 0.0f;
+    } else {
+        const float4 q = c.specBackground;
+        return q.x == 0.0f && q.y == 0.0f && q.z == 0.0f && q.w == 0.0f;
+    }
+}
+
 // Spectrum coefficients of the base colour and scatter radii of the material
 // at a hit, following resolveMaterial's albedo-texture rules.
 __device__ __forceinline__ void matCoefs(const DevScene& S, uint32_t mi, const pt_material& src, float u, float v,
@@ -637,19 +652,6 @@ __global__ void __launch_bounds__(256) k_generate(const LaunchCtx* __restrict__ 
 template <bool Count, bool Inst>
 #ifndef PT_EXTEND_MIN_BLOCKS
 #define PT_EXTEND_MIN_BLOCKS 4
-#endif
-#ifndef PT_SHADE_MIN_BLOCKS
-// (RGB shade at 4 blocks per SM, 64 registers: 8% less time per frame than at
-// 3 blocks and 80 registers on the 972k-triangle tree, 10% on the 64-tree
-// batch; the stage waits on dependent path-state and material loads, and the
-// fourth block hides more of that latency than the spills cost)
-#define PT_SHADE_MIN_BLOCKS 4
-#endif
-#ifndef PT_SHADE_SPEC_MIN_BLOCKS
-// (spectral shade at 4 blocks per SM, 64 registers: 531 -> 474 ms per frame on
-// the 972k-triangle tree with 8 wavelengths, each form on a grid of its own
-// occupancy)
-#define PT_SHADE_SPEC_MIN_BLOCKS 4
 #endif
 __global__ void __launch_bounds__(256, PT_EXTEND_MIN_BLOCKS) k_extend(const LaunchCtx* __restrict__ cp, int sel, bool identity, int iter)
 {
@@ -1018,8 +1020,25 @@ __global__ void __launch_bounds__(256, PT_SHADE_MISS_MIN_BLOCKS) k_shade_miss(co
 }
 
 // Shading of the paths that hit a triangle. One thread per queued path.
+//
+// Bound by instruction fetch: a path runs through about 30 KB of straight-line
+// code (the kernel has 170 - 230 KB), and with warps spread over it a third of
+// the stalls were fetches (issue slots 31% used, DRAM 26%; prefetching the next
+// path's state into shared memory changed nothing).  So the block's warps are
+// kept in phase by a barrier before each of the stretches below, and a block
+// is large: 16 warps share what one of them fetches.  Measured: hit shading of
+// the large frame (972k triangles, 1024^2, 256 spp, 8 wavelengths) 85.3 ms
+// without barriers, 68.5 with one per path, 64.7 with one at 512 threads, 60.6
+// with three (60.4 with five, which costs the forest view 4%); RGB: 6-tree
+// batch 11.3 -> 8.5 ms, zoo under a sky 4.9 -> 3.6 ms.
+constexpr int kShadeThreads = 512;
+#ifndef PT_SHADE_MIN_BLOCKS
+// (64 registers: at 3/4 of the warps and 80 registers the dependent loads of
+// path state and materials are hidden less than the spills cost)
+#define PT_SHADE_MIN_BLOCKS 2
+#endif
 template <int NW>
-__global__ void __launch_bounds__(256, NW == 0 ? PT_SHADE_MIN_BLOCKS : PT_SHADE_SPEC_MIN_BLOCKS)
+__global__ void __launch_bounds__(kShadeThreads, PT_SHADE_MIN_BLOCKS)
     k_shade(const LaunchCtx* __restrict__ cp, int sel, int iter)
 {
     const LaunchCtx& c = *cp;
@@ -1029,40 +1048,56 @@ __global__ void __launch_bounds__(256, NW == 0 ? PT_SHADE_MIN_BLOCKS : PT_SHADE_
     uint32_t* nextQueue = c.q.extend[sel ^ 1];
     const int debugFlags = c.params.brdf_debug_flags;
     const int cap = c.paths.capacity;
-    for (unsigned int k = blockIdx.x * blockDim.x + threadIdx.x; k < count; k += gridDim.x * blockDim.x) {
-        const uint32_t i = queue[k];
-        const DevScene& S = sceneOf(c, i);
-        const Waves<NW> wv = pathWaves<NW>(c, i);
-        const float4 r4 = c.paths.rad[i];
-        const int depth = __float_as_int(r4.w);
-        // RGB: the radiance stays in registers through the bounce.  Spectral: it
-        // is updated in memory (NEE of the previous bounce and the emission, in
-        // one read-modify-write below) and reloaded only by a path that ends.
-        Col<NW> L = czero<NW>();
-        if constexpr (NW == 0) {
-            L = loadCol<NW>(r4, c.paths.radS, cap, i);
-            // NEE contributions of the previous bounce, in the reference's order
-            // (the flags are clear for a path that starts at this bounce).
-            if (c.paths.visEnv[i]) {
-                L = cadd(L, pendingEnv<NW>(c, i));
-            }
-            if (c.paths.visEmis[i]) {
-                L = cadd(L, pendingEmis<NW>(c, i));
-            }
-        }
-        const float4 h4 = c.paths.hit[i];
-        const uint32_t tri = __float_as_uint(h4.w);
-        const float4 d4 = c.paths.dir[i];
-        const float3 d = f3(d4.x, d4.y, d4.z);
-        bool done = false;
+    // (the whole block runs the loop: barriers)
+    for (unsigned int base = blockIdx.x * blockDim.x; base < count; base += gridDim.x * blockDim.x) {
+        const unsigned int k = base + threadIdx.x;
+        const bool valid = k < count;
+        bool live = false; // hit below the depth limit
+        uint32_t i = 0u;
+        const DevScene* scene = &c.scene;
+        Waves<NW> wv{};
+        int depth = 0;
+        Col<NW> L, T, rho;
+        float4 r4, scatterCoef;
+        float3 d, pos, n;
+        float t = 0.0f, eta = 1.0f;
+        Ctx cx;
+        bool emitterMis = false, misVertex = false;
         bool pendEnv = false, pendEmis = false;
         bool cont = false;
-        if (depth >= c.maxDepth) {
-            done = true;
-        } else {
+        curandStateXORWOW st;
+        __syncthreads();
+        if (valid) {
+            i = queue[k];
+            scene = &sceneOf(c, i);
+            wv = pathWaves<NW>(c, i);
+            r4 = c.paths.rad[i];
+            depth = __float_as_int(r4.w);
+            // RGB: the radiance stays in registers through the bounce.  Spectral: it
+            // is updated in memory (NEE of the previous bounce and the emission, in
+            // one read-modify-write below) and reloaded only by a path that ends.
+            L = czero<NW>();
+            if constexpr (NW == 0) {
+                L = loadCol<NW>(r4, c.paths.radS, cap, i);
+                // NEE contributions of the previous bounce, in the reference's order
+                // (the flags are clear for a path that starts at this bounce).
+                if (c.paths.visEnv[i]) {
+                    L = cadd(L, pendingEnv<NW>(c, i));
+                }
+                if (c.paths.visEmis[i]) {
+                    L = cadd(L, pendingEmis<NW>(c, i));
+                }
+            }
+            live = depth < c.maxDepth;
+        }
+        const DevScene& S = *scene;
+        if (live) {
+            const float4 h4 = c.paths.hit[i];
+            const uint32_t tri = __float_as_uint(h4.w);
+            const float4 d4 = c.paths.dir[i];
+            d = f3(d4.x, d4.y, d4.z);
             const float4 o4 = c.paths.orig[i];
             const float4 t4 = c.paths.thr[i];
-            Col<NW> T;
             if constexpr (NW == 0) {
                 T = loadCol<NW>(t4, c.paths.thrS, cap, i);
             } else {
@@ -1075,12 +1110,11 @@ __global__ void __launch_bounds__(256, NW == 0 ? PT_SHADE_MIN_BLOCKS : PT_SHADE_
                     T = loadCol<NW>(t4, c.paths.thrS, cap, i);
                 }
             }
-            float eta = t4.w;
-            const float t = h4.x;
-            const float3 pos = xadd(f3(o4.x, o4.y, o4.z), xscl(d, t));
+            eta = t4.w;
+            t = h4.x;
+            pos = xadd(f3(o4.x, o4.y, o4.z), xscl(d, t));
             const float3 dn = xnormalize(d);
             const TriShade sh = S.shade[tri];
-            float3 n;
             float tu, tv;
             if (S.instanceCount == 0) {
                 hitShading(sh, dn, h4.y, h4.z, n, tu, tv);
@@ -1090,7 +1124,6 @@ __global__ void __launch_bounds__(256, NW == 0 ? PT_SHADE_MIN_BLOCKS : PT_SHADE_
             const uint32_t mi = __float_as_uint(sh.d.w);
             const pt_material& srcMat =
                 (S.materials != nullptr && mi < S.materialCount) ? S.materials[mi] : kFallbackMaterial;
-            Ctx cx;
             cx.m = resolveMaterial(srcMat, tu, tv, S.textures, S.textureCount);
             cx.w = computeLobes(cx.m);
             cx.n = n;
@@ -1101,8 +1134,8 @@ __global__ void __launch_bounds__(256, NW == 0 ? PT_SHADE_MIN_BLOCKS : PT_SHADE_
             // emissive NEE and the BSDF-sampled emitter hits share the light by the
             // balance heuristic, outside the transmit cones and above the surface;
             // elsewhere the reference's estimator is kept.
-            const bool emitterMis = c.params.emitter_mis == 1;
-            const bool misVertex = emitterMis && S.instanceCount == 0 && debugFlags == 0 && emitterMisVertex(cx);
+            emitterMis = c.params.emitter_mis == 1;
+            misVertex = emitterMis && S.instanceCount == 0 && debugFlags == 0 && emitterMisVertex(cx);
             // weight of this hit's emission: the previous vertex took part (pdf > 0) and
             // emissive NEE can pick this point (front face of a listed emitter)
             float emitW = 1.0f;
@@ -1121,8 +1154,7 @@ __global__ void __launch_bounds__(256, NW == 0 ? PT_SHADE_MIN_BLOCKS : PT_SHADE_
             }
             const float emission = cx.m.emission * emitW;
             // base colour at the path's wavelengths (spectral mode)
-            Col<NW> rho;
-            float4 scatterCoef = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            scatterCoef = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
             if constexpr (NW == 0) {
                 rho.c = f3(cx.m.r, cx.m.g, cx.m.b);
                 // emission (PathIntegratorRandCore.h:248)
@@ -1148,8 +1180,10 @@ __global__ void __launch_bounds__(256, NW == 0 ? PT_SHADE_MIN_BLOCKS : PT_SHADE_
                 }
                 storeCol<NW>(nullptr, c.paths.radS, cap, i, Lm, 0.0f);
             }
-            curandStateXORWOW st;
             rngLoad(c.paths, i, st);
+        }
+        __syncthreads();
+        if (live) {
             // environment NEE (PathIntegratorRandCore.h:65-108); with a distant
             // light, one more draw first picks the light or the environment
             if (!skipsEnvNee(cx.m)) {
@@ -1158,8 +1192,10 @@ __global__ void __launch_bounds__(256, NW == 0 ? PT_SHADE_MIN_BLOCKS : PT_SHADE_
                 const float u1 = curand_uniform(&st);
                 const float u2 = curand_uniform(&st);
                 float lp = 0.0f;
-                float3 wi;
-                if (!sunOn) {
+                float3 wi = f3(0.0f, 0.0f, 0.0f);
+                if (skyIsBlack<NW>(c)) {
+                    // (a light of exactly zero radiance adds nothing, whatever its sample)
+                } else if (!sunOn) {
                     wi = envSample(c.env, u1, u2, lp);
                 } else if (uSel < c.sun.select) {
                     wi = sunSample(c.sun, u1, u2);
@@ -1192,6 +1228,8 @@ __global__ void __launch_bounds__(256, NW == 0 ? PT_SHADE_MIN_BLOCKS : PT_SHADE_
                     }
                 }
             }
+        }
+        if (live) {
             // emissive NEE (PathIntegratorRandCore.h:110-167)
             if (S.emissiveCount > 0) {
                 const float uTri = curand_uniform(&st);
@@ -1259,13 +1297,15 @@ __global__ void __launch_bounds__(256, NW == 0 ? PT_SHADE_MIN_BLOCKS : PT_SHADE_
                     }
                 }
             }
+        }
+        __syncthreads();
+        if (live) {
             // BSDF sample (PathIntegratorRandCore.h:280-321)
             cx.debug = debugFlags;
             const float u1 = curand_uniform(&st);
             const float u2 = curand_uniform(&st);
             const BsdfSample smp = bsdfSample(cx, u1, u2);
             if (!smp.valid || smp.pdf <= kMinPdf) {
-                done = true;
             } else {
                 const Col<NW> f = evalCol<NW>(cx, smp.dir, rho, scatterCoef, wv);
                 T = throughCol<NW>(T, cx, smp, f, rho);
@@ -1295,8 +1335,7 @@ __global__ void __launch_bounds__(256, NW == 0 ? PT_SHADE_MIN_BLOCKS : PT_SHADE_
                 }
                 const float tl = pathWeight<NW>(T);
                 if (!isfinite(tl) || tl <= 0.0f || tl > 1.0e8f) {
-                    done = true;
-                } else {
+                    } else {
                     bool survive = true;
                     if (depth >= c.rrMinDepth) {
                         const float surv = fmin2(0.95f, fmax2(tl, 0.05f));
@@ -1307,8 +1346,7 @@ __global__ void __launch_bounds__(256, NW == 0 ? PT_SHADE_MIN_BLOCKS : PT_SHADE_
                         }
                     }
                     if (!survive) {
-                        done = true;
-                    } else {
+                            } else {
                         eta = smp.nextEta;
                         const float bias = fmax2(1.0e-4f, 1.0e-3f * t);
                         const float sign = dot3(n, smp.dir) >= 0.0f ? 1.0f : -1.0f;
@@ -1327,47 +1365,48 @@ __global__ void __launch_bounds__(256, NW == 0 ? PT_SHADE_MIN_BLOCKS : PT_SHADE_
             }
             rngStore(c.paths, i, st);
         }
-        (void)done;
-        if constexpr (NW == 0) {
-            c.paths.visEnv[i] = 0;
-            c.paths.visEmis[i] = 0;
-            if (cont) {
-                storeCol<NW>(c.paths.rad, c.paths.radS, cap, i, L, __int_as_float(depth + 1));
-                queueNext(c, i, nextCount, nextQueue);
-            } else if (pendEnv || pendEmis) {
-                storeCol<NW>(c.paths.rad, c.paths.radS, cap, i, L, __int_as_float(depth));
-                const uint32_t s = warpPush(&c.q.counts[3]);
-                c.q.finish[s] = i;
-            } else {
-                writeSample<NW>(c, i, L, wv);
-                recyclePath<NW>(c, i, nextCount, nextQueue);
-            }
-        } else {
-            if (cont || pendEnv || pendEmis) {
-                // the radiance is in radS already
-                c.paths.rad[i] = make_float4(0.0f, 0.0f, 0.0f, __int_as_float(cont ? depth + 1 : depth));
+        if (valid) {
+            if constexpr (NW == 0) {
+                c.paths.visEnv[i] = 0;
+                c.paths.visEmis[i] = 0;
                 if (cont) {
+                    storeCol<NW>(c.paths.rad, c.paths.radS, cap, i, L, __int_as_float(depth + 1));
                     queueNext(c, i, nextCount, nextQueue);
-                } else {
+                } else if (pendEnv || pendEmis) {
+                    storeCol<NW>(c.paths.rad, c.paths.radS, cap, i, L, __int_as_float(depth));
                     const uint32_t s = warpPush(&c.q.counts[3]);
                     c.q.finish[s] = i;
+                } else {
+                    writeSample<NW>(c, i, L, wv);
+                    recyclePath<NW>(c, i, nextCount, nextQueue);
                 }
             } else {
-                L = loadCol<NW>(r4, c.paths.radS, cap, i);
-                if (depth >= c.maxDepth) {
-                    // (no read-modify-write happened: add the previous bounce's NEE here)
-                    if (c.paths.visEnv[i]) {
-                        L = cadd(L, pendingEnv<NW>(c, i));
+                if (cont || pendEnv || pendEmis) {
+                    // the radiance is in radS already
+                    c.paths.rad[i] = make_float4(0.0f, 0.0f, 0.0f, __int_as_float(cont ? depth + 1 : depth));
+                    if (cont) {
+                        queueNext(c, i, nextCount, nextQueue);
+                    } else {
+                        const uint32_t s = warpPush(&c.q.counts[3]);
+                        c.q.finish[s] = i;
                     }
-                    if (c.paths.visEmis[i]) {
-                        L = cadd(L, pendingEmis<NW>(c, i));
+                } else {
+                    L = loadCol<NW>(r4, c.paths.radS, cap, i);
+                    if (depth >= c.maxDepth) {
+                        // (no read-modify-write happened: add the previous bounce's NEE here)
+                        if (c.paths.visEnv[i]) {
+                            L = cadd(L, pendingEnv<NW>(c, i));
+                        }
+                        if (c.paths.visEmis[i]) {
+                            L = cadd(L, pendingEmis<NW>(c, i));
+                        }
                     }
+                    writeSample<NW>(c, i, L, wv);
+                    recyclePath<NW>(c, i, nextCount, nextQueue);
                 }
-                writeSample<NW>(c, i, L, wv);
-                recyclePath<NW>(c, i, nextCount, nextQueue);
+                c.paths.visEnv[i] = 0;
+                c.paths.visEmis[i] = 0;
             }
-            c.paths.visEnv[i] = 0;
-            c.paths.visEmis[i] = 0;
         }
     }
 }
@@ -1756,11 +1795,11 @@ void launchShadeMiss(const LaunchCtx* c, int iter, int sel, int grid, int nw, cu
 void launchShade(const LaunchCtx* c, int sel, int iter, int grid, int nw, cudaStream_t s)
 {
     if (nw == 8) {
-        k_shade<8><<<grid, 256, 0, s>>>(c, sel, iter);
+        k_shade<8><<<grid, kShadeThreads, 0, s>>>(c, sel, iter);
     } else if (nw == 4) {
-        k_shade<4><<<grid, 256, 0, s>>>(c, sel, iter);
+        k_shade<4><<<grid, kShadeThreads, 0, s>>>(c, sel, iter);
     } else {
-        k_shade<0><<<grid, 256, 0, s>>>(c, sel, iter);
+        k_shade<0><<<grid, kShadeThreads, 0, s>>>(c, sel, iter);
     }
 }
 void launchShadow(const LaunchCtx* c, int iter, int grid, bool count, bool inst, bool lane, bool multi, cudaStream_t s)
@@ -1797,11 +1836,11 @@ int shadeOccupancy(int nw)
     if (occ[k].load(std::memory_order_relaxed) == 0) {
         int b = 1;
         if (nw == 8) {
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_shade<8>, 256, 0);
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_shade<8>, kShadeThreads, 0);
         } else if (nw == 4) {
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_shade<4>, 256, 0);
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_shade<4>, kShadeThreads, 0);
         } else {
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_shade<0>, 256, 0);
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_shade<0>, kShadeThreads, 0);
         }
         occ[k].store(b > 0 ? b : 1, std::memory_order_relaxed);
     }
@@ -1812,7 +1851,7 @@ void stageOccupancy(int& extendBlocks, int& shadeBlocks, int& shadowBlocks)
     extendBlocks = shadeBlocks = shadowBlocks = 1;
     const size_t smem = sizeof(uint2) * kSharedStack * 256;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&extendBlocks, k_extend<false, false>, 256, smem);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&shadeBlocks, k_shade<0>, 256, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&shadeBlocks, k_shade<0>, kShadeThreads, 0);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&shadowBlocks, k_shadow<false, false>, 256, smem);
 }
 void launchFinalize(const LaunchCtx* c, int sel, int grid, int nw, cudaStream_t s)
