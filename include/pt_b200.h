@@ -269,11 +269,10 @@ int pt_get_profile(const pt_renderer* r, pt_profile* out);
 int pt_set_tuning(pt_renderer* r, int path_capacity, int blocks_per_sm);
 
 /* Closest-hit and shadow-ray scheduling (no reference counterpart; images are
- * identical in every mode).  AUTO: per-lane ray replacement (closest hit and
- * shadow rays; two-level traversal in instanced scenes) with a slot-ordered
- * next-bounce queue when the largest flat scene or instanced object has at
- * least 32768 BVH nodes, else one warp per 32 queued rays.  WARP / LANE force
- * either form. */
+ * identical in every mode).  AUTO and LANE: whole-warp traversal with ray
+ * replacement (closest hit and shadow rays; two-level traversal in instanced
+ * scenes) and a slot-ordered next-bounce queue.  WARP: one warp per 32 queued
+ * rays, each lane on its own. */
 enum pt_extend_mode { PT_EXTEND_MODE_AUTO = 0, PT_EXTEND_MODE_WARP = 1, PT_EXTEND_MODE_LANE = 2 };
 int pt_set_extend_mode(pt_renderer* r, int mode);
 

@@ -1224,10 +1224,6 @@ void releaseBounceGraphs(pt_renderer* r)
     }
 }
 
-#ifndef PT_EXTEND_LANE_MIN_NODES
-#define PT_EXTEND_LANE_MIN_NODES 32768
-#endif
-
 // Grid of the closest-hit stage: the per-lane kernel has its own occupancy.
 int extendGrid(const pt_renderer* r, bool count, bool inst)
 {
@@ -1643,19 +1639,13 @@ int pt_render(pt_renderer* r, int waves)
         }
     }
     bool inst = false;
-    uint32_t maxNodes = 0;
     for (const SceneSlot& sl : r->scenes) {
         inst = inst || sl.instanceCount > 0;
-        maxNodes = std::max(maxNodes, sl.bvh.nodeCount);
-        for (const BvhBuffers& b : sl.objBvh) {
-            maxNodes = std::max(maxNodes, b.nodeCount); // an instanced scene's objects
-        }
     }
-    // Per-lane ray replacement pays where traversals are long (large trees, and
-    // instanced scenes of large objects: the two-level traversal); on small
-    // scenes the extra routing launch costs more than it saves.
-    r->extendLane = r->extendMode == PT_EXTEND_MODE_LANE ||
-        (r->extendMode == PT_EXTEND_MODE_AUTO && maxNodes >= static_cast<uint32_t>(PT_EXTEND_LANE_MIN_NODES));
+    // The whole-warp traversal, its routing and its slot-ordered queues are the
+    // better form for every size of scene (2.4k triangles, 641x359, 16 spp: closest
+    // hit 7.0 -> 3.7 ms; 20k triangles, 96x64, one sample: even).
+    r->extendLane = r->extendMode != PT_EXTEND_MODE_WARP;
     const int nw = r->params.spectral_wavelengths;
     if (nw > 0) {
         const int st = prepareSpectral(r, nw);

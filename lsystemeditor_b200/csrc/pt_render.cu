@@ -838,142 +838,211 @@ static __device__ __noinline__ uint32_t routeQ1(const LaunchCtx& c, uint32_t i)
 }
 
 // Splits the queue that k_extend_lane marked into the miss and hit queues of
-// this bounce, in queue order.  A block takes a tile of 8 x 256 consecutive
-// entries, counts its hits and misses per warp and row (ballots), reserves
-// both output ranges with one atomic each, and writes every entry to its rank
-// within the tile: two atomics per 2048 entries instead of two per warp.
-constexpr int kRouteRows = 8;
-// (blocks of 256 threads = 8 warps; warp 0 scans the 64 (row, warp) counts, two per lane)
-static_assert(kRouteRows * 8 == 64, "the tile scan covers exactly 64 (row, warp) counts");
-__global__ void __launch_bounds__(256) k_route(const LaunchCtx* __restrict__ cp, int sel, int iter)
+// this bounce.  Every warp takes one contiguous part of the queue, counts its
+// hits, the block reserves both output ranges with one atomic each, and the
+// warp reads its part again and writes it in order.  Bound by the atomics when
+// a tile of 2048 entries had two of its own (they serialise on one address,
+// about 10 ns each): 16.7M entries 162 -> 56 us, below 1M entries unchanged.
+constexpr int kListThreads = 256;
+constexpr int kListWarps = kListThreads / 32;
+constexpr int kRouteRows = 8; // loads in flight per lane
+
+__global__ void __launch_bounds__(kListThreads) k_route(const LaunchCtx* __restrict__ cp, int sel, int iter)
 {
     const LaunchCtx& c = *cp;
     const unsigned int count = c.q.counts[sel];
     const int par = iter & 1;
     uint32_t* queue = c.q.extend[sel];
-    const bool q1 = c.q.counts[12 + par] != 0u;
-    __shared__ unsigned int sHit[kRouteRows * 8], sMiss[kRouteRows * 8]; // exclusive offsets per (row, warp)
-    __shared__ unsigned int sBase[2];
+    __shared__ unsigned int sHit[kListWarps], sMiss[kListWarps]; // counts, then first output positions
     const unsigned int lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const unsigned int below = (1u << lane) - 1u;
-    const unsigned int tile = 256u * kRouteRows;
-    for (unsigned int t0 = blockIdx.x * tile; t0 < count; t0 += gridDim.x * tile) {
-        if (q1) {
-            for (unsigned int k = t0 + threadIdx.x; k < min(t0 + tile, count); k += 256u) {
-                if ((queue[k] & 0x40000000u) != 0u) {
-                    queue[k] = routeQ1(c, queue[k] & 0x3FFFFFFFu);
-                }
+    const unsigned int warps = gridDim.x * kListWarps;
+    const unsigned int part = ((count + warps - 1u) / warps + 31u) & ~31u;
+    if (blockIdx.x * kListWarps * part >= count) {
+        return;
+    }
+    const unsigned int first = min((blockIdx.x * kListWarps + warp) * part, count), last = min(first + part, count);
+    if (c.q.counts[12 + par] != 0u) {
+        for (unsigned int k = first + lane; k < last; k += 32u) {
+            if ((queue[k] & 0x40000000u) != 0u) {
+                queue[k] = routeQ1(c, queue[k] & 0x3FFFFFFFu);
             }
         }
+    }
+    // (a lane reads the entries that it wrote)
+    unsigned int hits = 0;
+#pragma unroll kRouteRows
+    for (unsigned int k = first + lane; k < last; k += 32u) {
+        hits += 1u - (queue[k] >> 31);
+    }
+    hits = __reduce_add_sync(0xffffffffu, hits);
+    if (lane == 0) {
+        sHit[warp] = hits;
+        sMiss[warp] = last - first - hits;
+    }
+    __syncthreads();
+    if (warp == 0) {
+        const unsigned int h = lane < kListWarps ? sHit[lane] : 0u, m = lane < kListWarps ? sMiss[lane] : 0u;
+        unsigned int hs = h, ms = m;
+#pragma unroll
+        for (int d = 1; d < kListWarps; d <<= 1) {
+            const unsigned int ho = __shfl_up_sync(0xffffffffu, hs, d);
+            const unsigned int mo = __shfl_up_sync(0xffffffffu, ms, d);
+            if (lane >= static_cast<unsigned int>(d)) {
+                hs += ho;
+                ms += mo;
+            }
+        }
+        // (the last warp's lane holds the totals)
+        unsigned int hb = 0, mb = 0;
+        if (lane == kListWarps - 1) {
+            hb = hs != 0u ? atomicAdd(&c.q.counts[5 + 2 * par], hs) : 0u;
+            mb = ms != 0u ? atomicAdd(&c.q.counts[4 + 2 * par], ms) : 0u;
+        }
+        hb = __shfl_sync(0xffffffffu, hb, kListWarps - 1);
+        mb = __shfl_sync(0xffffffffu, mb, kListWarps - 1);
+        if (lane < kListWarps) {
+            sHit[lane] = hb + hs - h;
+            sMiss[lane] = mb + ms - m;
+        }
+    }
+    __syncthreads();
+    unsigned int hitAt = sHit[warp], missAt = sMiss[warp];
+    for (unsigned int k0 = first; k0 < last; k0 += 32u * kRouteRows) {
         uint32_t e[kRouteRows];
-        unsigned int hitMask[kRouteRows], missMask[kRouteRows];
 #pragma unroll
         for (int r = 0; r < kRouteRows; ++r) {
-            const unsigned int k = t0 + static_cast<unsigned int>(r) * 256u + threadIdx.x;
-            const bool valid = k < count;
-            e[r] = valid ? queue[k] : 0u;
-            const bool miss = valid && (e[r] & 0x80000000u) != 0u;
-            hitMask[r] = __ballot_sync(0xffffffffu, valid && !miss);
-            missMask[r] = __ballot_sync(0xffffffffu, miss);
-            if (lane == 0) {
-                sHit[r * 8 + warp] = __popc(hitMask[r]);
-                sMiss[r * 8 + warp] = __popc(missMask[r]);
-            }
+            const unsigned int k = k0 + static_cast<unsigned int>(r) * 32u + lane;
+            e[r] = k < last ? queue[k] : 0u;
         }
-        __syncthreads();
-        if (warp == 0) {
-            // exclusive scan of the 64 (row, warp) counts in queue order, two per lane
-            const unsigned int h0 = sHit[2 * lane], h1 = sHit[2 * lane + 1];
-            const unsigned int m0 = sMiss[2 * lane], m1 = sMiss[2 * lane + 1];
-            unsigned int h = h0 + h1, m = m0 + m1;
 #pragma unroll
-            for (int d = 1; d < 32; d <<= 1) {
-                const unsigned int ho = __shfl_up_sync(0xffffffffu, h, d);
-                const unsigned int mo = __shfl_up_sync(0xffffffffu, m, d);
-                if (lane >= static_cast<unsigned int>(d)) {
-                    h += ho;
-                    m += mo;
+        for (int r = 0; r < kRouteRows; ++r) {
+            const bool valid = k0 + static_cast<unsigned int>(r) * 32u + lane < last;
+            const bool miss = (e[r] >> 31) != 0u;
+            const unsigned int hm = __ballot_sync(0xffffffffu, valid && !miss);
+            const unsigned int mm = __ballot_sync(0xffffffffu, valid && miss);
+            if (valid) {
+                if (miss) {
+                    c.q.missQueue[missAt + __popc(mm & below)] = e[r] & 0x7FFFFFFFu;
+                } else {
+                    c.q.hitQueue[hitAt + __popc(hm & below)] = e[r];
                 }
             }
-            const unsigned int hTot = __shfl_sync(0xffffffffu, h, 31), mTot = __shfl_sync(0xffffffffu, m, 31);
-            sHit[2 * lane] = h - h0 - h1;
-            sHit[2 * lane + 1] = h - h1;
-            sMiss[2 * lane] = m - m0 - m1;
-            sMiss[2 * lane + 1] = m - m1;
-            if (lane == 0) {
-                sBase[0] = hTot ? atomicAdd(&c.q.counts[5 + 2 * par], hTot) : 0u;
-                sBase[1] = mTot ? atomicAdd(&c.q.counts[4 + 2 * par], mTot) : 0u;
-            }
+            hitAt += __popc(hm);
+            missAt += __popc(mm);
         }
-        __syncthreads();
-#pragma unroll
-        for (int r = 0; r < kRouteRows; ++r) {
-            if ((hitMask[r] >> lane) & 1u) {
-                c.q.hitQueue[sBase[0] + sHit[r * 8 + warp] + __popc(hitMask[r] & below)] = e[r];
-            } else if ((missMask[r] >> lane) & 1u) {
-                c.q.missQueue[sBase[1] + sMiss[r * 8 + warp] + __popc(missMask[r] & below)] = e[r] & 0x7FFFFFFFu;
-            }
-        }
-        __syncthreads(); // the shared offsets are rewritten by the next tile
     }
 }
 
-// Slot-ordered mode: lists the slots the shade kernels marked as the next
-// bounce's extend queue, in increasing slot order within tiles of 2048 (the
-// tiles in the order they reserve their ranges), and clears the marks.  The
-// extend and shade kernels then read the path state of consecutive slots.
-__global__ void __launch_bounds__(256) k_next_queue(const LaunchCtx* __restrict__ cp, int sel)
+// Slot-ordered mode: lists the slots the shade kernels marked (bytes of 0 or
+// 1) as the next bounce's extend queue and clears the marks.  Every warp takes
+// one contiguous range of slots, 16 marks per load, as in k_route, so that the
+// extend and shade kernels read the path state of consecutive slots.  One mark
+// per load kept 8 KB per SM in flight: 16.7M slots 78 -> 22 us (69 -> 9 with
+// no slot marked).
+constexpr unsigned int kMarksPerRow = 512; // slots of one step of a warp
+__device__ __forceinline__ uint4 loadMarks(const uint8_t* flag, unsigned int k, unsigned int n)
+{
+    if (k + 16u <= n) {
+        return *reinterpret_cast<const uint4*>(flag + k);
+    }
+    uint32_t w[4] = {0u, 0u, 0u, 0u};
+    for (unsigned int j = 0; k + j < n; ++j) {
+        w[j >> 2] |= static_cast<uint32_t>(flag[k + j]) << (8u * (j & 3u));
+    }
+    return make_uint4(w[0], w[1], w[2], w[3]);
+}
+__global__ void __launch_bounds__(kListThreads) k_next_queue(const LaunchCtx* __restrict__ cp, int sel)
 {
     const LaunchCtx& c = *cp;
     const unsigned int n = static_cast<unsigned int>(c.q.batch->slotCount);
     uint8_t* flag = c.q.nextFlag;
     uint32_t* out = c.q.extend[sel ^ 1];
-    __shared__ unsigned int sOff[kRouteRows * 8];
-    __shared__ unsigned int sBase;
+    __shared__ unsigned int sAt[kListWarps]; // counts, then first output positions
+    __shared__ uint16_t sSlot[kListWarps][kMarksPerRow];
     const unsigned int lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    const unsigned int below = (1u << lane) - 1u;
-    const unsigned int tile = 256u * kRouteRows;
-    for (unsigned int t0 = blockIdx.x * tile; t0 < n; t0 += gridDim.x * tile) {
-        unsigned int mask[kRouteRows];
+    const unsigned int warps = gridDim.x * kListWarps;
+    const unsigned int part = ((n + warps - 1u) / warps + kMarksPerRow - 1u) / kMarksPerRow * kMarksPerRow;
+    if (blockIdx.x * kListWarps * part >= n) {
+        return;
+    }
+    const unsigned int first = min((blockIdx.x * kListWarps + warp) * part, n), last = min(first + part, n);
+    unsigned int marks = 0;
+#pragma unroll 4
+    for (unsigned int k = first + 16u * lane; k < last; k += kMarksPerRow) {
+        const uint4 v = loadMarks(flag, k, last);
+        // (bytes are 0 or 1: the four words' bits do not meet)
+        marks += __popc(v.x | (v.y << 1) | (v.z << 2) | (v.w << 3));
+    }
+    marks = __reduce_add_sync(0xffffffffu, marks);
+    if (lane == 0) {
+        sAt[warp] = marks;
+    }
+    __syncthreads();
+    if (warp == 0) {
+        const unsigned int a = lane < kListWarps ? sAt[lane] : 0u;
+        unsigned int s = a;
 #pragma unroll
-        for (int r = 0; r < kRouteRows; ++r) {
-            const unsigned int k = t0 + static_cast<unsigned int>(r) * 256u + threadIdx.x;
-            const bool on = k < n && flag[k] != 0;
-            if (on) {
-                flag[k] = 0;
-            }
-            mask[r] = __ballot_sync(0xffffffffu, on);
-            if (lane == 0) {
-                sOff[r * 8 + warp] = __popc(mask[r]);
+        for (int d = 1; d < kListWarps; d <<= 1) {
+            const unsigned int o = __shfl_up_sync(0xffffffffu, s, d);
+            if (lane >= static_cast<unsigned int>(d)) {
+                s += o;
             }
         }
-        __syncthreads();
-        if (warp == 0) {
-            const unsigned int a0 = sOff[2 * lane], a1 = sOff[2 * lane + 1];
-            unsigned int a = a0 + a1;
+        unsigned int b = 0;
+        if (lane == kListWarps - 1 && s != 0u) {
+            b = atomicAdd(&c.q.counts[sel ^ 1], s);
+        }
+        b = __shfl_sync(0xffffffffu, b, kListWarps - 1);
+        if (lane < kListWarps) {
+            sAt[lane] = b + s - a;
+        }
+    }
+    __syncthreads();
+    if (marks == 0u) {
+        return;
+    }
+    unsigned int at = sAt[warp];
+    uint16_t* slots = sSlot[warp];
+    for (unsigned int k0 = first; k0 < last; k0 += kMarksPerRow) {
+        const unsigned int k = k0 + 16u * lane;
+        const uint4 v = k < last ? loadMarks(flag, k, last) : make_uint4(0u, 0u, 0u, 0u);
+        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+        const unsigned int own = __popc(v.x | (v.y << 1) | (v.z << 2) | (v.w << 3));
+        unsigned int s = own;
 #pragma unroll
-            for (int d = 1; d < 32; d <<= 1) {
-                const unsigned int o = __shfl_up_sync(0xffffffffu, a, d);
-                if (lane >= static_cast<unsigned int>(d)) {
-                    a += o;
+        for (int d = 1; d < 32; d <<= 1) {
+            const unsigned int o = __shfl_up_sync(0xffffffffu, s, d);
+            if (lane >= static_cast<unsigned int>(d)) {
+                s += o;
+            }
+        }
+        const unsigned int total = __shfl_sync(0xffffffffu, s, 31);
+        if (total == 0u) {
+            continue;
+        }
+        unsigned int o = s - own;
+#pragma unroll
+        for (unsigned int j = 0; j < 16u; ++j) {
+            if (((w[j >> 2] >> (8u * (j & 3u))) & 1u) != 0u) {
+                slots[o++] = static_cast<uint16_t>(16u * lane + j);
+            }
+        }
+        if (own != 0u) {
+            if (k + 16u <= last) {
+                *reinterpret_cast<uint4*>(flag + k) = make_uint4(0u, 0u, 0u, 0u);
+            } else {
+                for (unsigned int j = 0; k + j < last; ++j) {
+                    flag[k + j] = 0;
                 }
             }
-            const unsigned int tot = __shfl_sync(0xffffffffu, a, 31);
-            sOff[2 * lane] = a - a0 - a1;
-            sOff[2 * lane + 1] = a - a1;
-            if (lane == 0) {
-                sBase = tot ? atomicAdd(&c.q.counts[sel ^ 1], tot) : 0u;
-            }
         }
-        __syncthreads();
-#pragma unroll
-        for (int r = 0; r < kRouteRows; ++r) {
-            if ((mask[r] >> lane) & 1u) {
-                out[sBase + sOff[r * 8 + warp] + __popc(mask[r] & below)] =
-                    t0 + static_cast<unsigned int>(r) * 256u + threadIdx.x;
-            }
+        __syncwarp();
+        for (unsigned int q = lane; q < total; q += 32u) {
+            out[at + q] = k0 + slots[q];
         }
-        __syncthreads();
+        __syncwarp(); // the list is rewritten by the next step
+        at += total;
     }
 }
 
@@ -998,8 +1067,9 @@ __global__ void __launch_bounds__(256, PT_SHADE_MISS_MIN_BLOCKS) k_shade_miss(co
         const int depth = __float_as_int(r4.w);
         Col<NW> L;
         const bool sunOn = c.sun.enabled != 0;
+        const bool black = skyIsBlack<NW>(c); // (adds exactly nothing)
         if (depth == 0) {
-            L = sunOn ? skyCol<NW>(c, d, wv) : envCol<NW>(c, d, wv);
+            L = black ? czero<NW>() : sunOn ? skyCol<NW>(c, d, wv) : envCol<NW>(c, d, wv);
         } else {
             L = loadCol<NW>(r4, c.paths.radS, c.paths.capacity, i);
             if (c.paths.visEnv[i]) {
@@ -1008,11 +1078,13 @@ __global__ void __launch_bounds__(256, PT_SHADE_MISS_MIN_BLOCKS) k_shade_miss(co
             if (c.paths.visEmis[i]) {
                 L = cadd(L, pendingEmis<NW>(c, i));
             }
-            const Col<NW> T = loadCol<NW>(c.paths.thr[i], c.paths.thrS, c.paths.capacity, i);
-            const Col<NW> Le = sunOn ? skyCol<NW>(c, d, wv) : envCol<NW>(c, d, wv);
-            const float lp = sunOn ? skyPdf(c, d) : envPdf(c.env, d);
-            const float w = misBalance(fabsf(d4.w), lp);
-            L = cadd(L, cmul(T, cscl(Le, w)));
+            if (!black) {
+                const Col<NW> T = loadCol<NW>(c.paths.thr[i], c.paths.thrS, c.paths.capacity, i);
+                const Col<NW> Le = sunOn ? skyCol<NW>(c, d, wv) : envCol<NW>(c, d, wv);
+                const float lp = sunOn ? skyPdf(c, d) : envPdf(c.env, d);
+                const float w = misBalance(fabsf(d4.w), lp);
+                L = cadd(L, cmul(T, cscl(Le, w)));
+            }
         }
         writeSample<NW>(c, i, L, wv);
         recyclePath<NW>(c, i, nextCount, nextQueue);
@@ -1739,7 +1811,7 @@ void launchExtend(const LaunchCtx* c, int sel, bool identity, int iter, int grid
         } else {
             k_extend_lane<false, false><<<grid, kTraceThreads, traceSmemBytes<false>(), s>>>(c, sel, identity, iter);
         }
-        k_route<<<grid, 256, 0, s>>>(c, sel, iter);
+        k_route<<<grid, kListThreads, 0, s>>>(c, sel, iter);
     } else if (inst) {
         if (count) {
             k_extend<true, true><<<grid, 256, smem, s>>>(c, sel, identity, iter);
@@ -1758,7 +1830,7 @@ int extendKernels(bool count, bool inst, bool lane)
 }
 void launchNextQueue(const LaunchCtx* c, int sel, int grid, cudaStream_t s)
 {
-    k_next_queue<<<grid, 256, 0, s>>>(c, sel);
+    k_next_queue<<<grid, kListThreads, 0, s>>>(c, sel);
 }
 int extendLaneOccupancy()
 {

@@ -114,10 +114,12 @@ __device__ __forceinline__ void warpTraversal(const DevScene& S0, unsigned int c
     const TriVerts* tris = Inst ? nullptr : S0.tris;
     int level = 0, base = 0;
     // the warp's chunk of the queue; small queues are spread over all warps
-    unsigned int poolNext = 0, poolEnd = 0;
-    bool drained = false;
+    // (a warp's first chunk is its own; the counter hands out those behind them)
     const unsigned int warps = gridDim.x * (kTraceThreads / 32);
     const unsigned int chunk = min(kTraceChunk, max(1u, count / (warps * 2u)));
+    unsigned int poolNext = (blockIdx.x * (kTraceThreads / 32) + (threadIdx.x >> 5)) * chunk;
+    unsigned int poolEnd = min(poolNext + chunk, count);
+    bool drained = poolNext >= count;
 
     auto push = [&](uint2 g) -> bool {
         if (sp < kTraceStack) {
@@ -150,7 +152,7 @@ __device__ __forceinline__ void warpTraversal(const DevScene& S0, unsigned int c
                 if (lane == 0) {
                     b = atomicAdd(fetch, chunk);
                 }
-                poolNext = __shfl_sync(kAll, b, 0);
+                poolNext = __shfl_sync(kAll, b, 0) + warps * chunk;
                 poolEnd = min(poolNext + chunk, count);
                 drained = poolNext >= count;
             }

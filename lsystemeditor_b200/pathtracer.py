@@ -610,7 +610,7 @@ class PathTracer:
         return float(c.value)
 
     def set_extend_mode(self, mode: int):
-        """pt_set_extend_mode: 0 auto, 1 warp-fetch closest hit, 2 per-lane replacement (identical images)."""
+        """pt_set_extend_mode: 0 auto, 1 one ray per lane, 2 whole-warp traversal, as auto (identical images)."""
         self._check(self._lib.pt_set_extend_mode(self._h, int(mode)))
 
     def rng_tape(self, first_wave: int, waves: int, stride: int) -> np.ndarray:
