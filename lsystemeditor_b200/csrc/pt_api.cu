@@ -120,7 +120,6 @@ struct SceneSlot {
         specValid = false;
         releaseInstances();
         bvh.nodeCount = bvh.triCount = 0;
-        bvh.levels = 0;
         shareFrom = -1;
         triCount = materialCount = textureCount = emissiveCount = 0;
         hasScene = false;

@@ -21,6 +21,7 @@
 #include "pt_bvh.cuh"
 
 
+#include <algorithm>
 #include <cfloat>
 #include <cmath>
 #include <cstdio>
@@ -63,7 +64,8 @@ __global__ void k_prepare(const float* __restrict__ pos, uint32_t n, float4* __r
         cmin = make_float3(fminf(cmin.x, ce.x), fminf(cmin.y, ce.y), fminf(cmin.z, ce.z));
         cmax = make_float3(fmaxf(cmax.x, ce.x), fmaxf(cmax.y, ce.y), fmaxf(cmax.z, ce.z));
     }
-    // warp reduce, then one atomic per warp
+    // warp and block reductions, then one atomic per block and bound (an atomic
+    // per warp was 182k on six addresses for 972k triangles: 129 -> 13 us)
     for (int off = 16; off > 0; off >>= 1) {
         cmin.x = fminf(cmin.x, __shfl_xor_sync(0xffffffffu, cmin.x, off));
         cmin.y = fminf(cmin.y, __shfl_xor_sync(0xffffffffu, cmin.y, off));
@@ -72,13 +74,27 @@ __global__ void k_prepare(const float* __restrict__ pos, uint32_t n, float4* __r
         cmax.y = fmaxf(cmax.y, __shfl_xor_sync(0xffffffffu, cmax.y, off));
         cmax.z = fmaxf(cmax.z, __shfl_xor_sync(0xffffffffu, cmax.z, off));
     }
+    __shared__ float sBound[6][kBlock / 32];
     if ((threadIdx.x & 31) == 0) {
-        atomicMin(&cbounds[0], floatToOrdered(cmin.x));
-        atomicMin(&cbounds[1], floatToOrdered(cmin.y));
-        atomicMin(&cbounds[2], floatToOrdered(cmin.z));
-        atomicMax(&cbounds[3], floatToOrdered(cmax.x));
-        atomicMax(&cbounds[4], floatToOrdered(cmax.y));
-        atomicMax(&cbounds[5], floatToOrdered(cmax.z));
+        const int w = threadIdx.x >> 5;
+        sBound[0][w] = cmin.x;
+        sBound[1][w] = cmin.y;
+        sBound[2][w] = cmin.z;
+        sBound[3][w] = cmax.x;
+        sBound[4][w] = cmax.y;
+        sBound[5][w] = cmax.z;
+    }
+    __syncthreads();
+    if (threadIdx.x < 6) {
+        float v = sBound[threadIdx.x][0];
+        for (int w = 1; w < kBlock / 32; ++w) {
+            v = threadIdx.x < 3 ? fminf(v, sBound[threadIdx.x][w]) : fmaxf(v, sBound[threadIdx.x][w]);
+        }
+        if (threadIdx.x < 3) {
+            atomicMin(&cbounds[threadIdx.x], floatToOrdered(v));
+        } else {
+            atomicMax(&cbounds[threadIdx.x], floatToOrdered(v));
+        }
     }
 }
 
@@ -212,157 +228,307 @@ __device__ __forceinline__ float boxArea(float3 lo, float3 hi)
 // cost, and the treelet is rewritten in place. Processed bottom-up, one
 // treelet per warp, with visit counters like k_refit so that a node is
 // optimised only after both subtrees are final.
+//
+// Bound by latency: a treelet is a chain of dependent loads, and the treelets
+// towards the root are a chain themselves.  So lane k holds treelet leaf k (one
+// round trip per opened leaf: its box, children and cost are loaded together),
+// the subsets' boxes come from the seven leaf boxes in shared memory, and the
+// partitions of the two largest subset sizes are spread over the lanes.  The
+// first form (one lane forming the treelet, boxes read from L2 per subset, one
+// lane per subset) took 4.96 ms for 972k triangles and 1.90 ms for 132k; this
+// one 1.10 and 0.48 ms.  Same trees.
 constexpr int kTreeletLeaves = 7;
 constexpr int kSubsets = 1 << kTreeletLeaves;
 
 struct TreeletScratch {
     float area[kSubsets];
     float cost[kSubsets];
+    float4 leafLo[kTreeletLeaves]; // w: triangles (int bits)
+    float4 leafHi[kTreeletLeaves];
+    int leaf[kTreeletLeaves];
+    int internal[kTreeletLeaves - 1];
+    int kids[kTreeletLeaves - 1][2]; // of the rewritten internal nodes
+    uint8_t mask[kTreeletLeaves - 1]; // their leaf subsets
     uint8_t split[kSubsets];
-    float4 lo[kSubsets];
-    float4 hi[kSubsets];
 };
+
+// Subsets of seven leaves by size: 2 (21 of them), 3 (35), 4 (35), 5 (21).
+struct SubsetTable {
+    uint8_t m[112];
+};
+constexpr SubsetTable makeSubsetTable()
+{
+    SubsetTable t{};
+    int at = 0;
+    for (int size = 2; size <= 5; ++size) {
+        for (int m = 1; m < kSubsets; ++m) {
+            int bits = 0;
+            for (int k = 0; k < kTreeletLeaves; ++k) {
+                bits += (m >> k) & 1;
+            }
+            if (bits == size) {
+                t.m[at++] = static_cast<uint8_t>(m);
+            }
+        }
+    }
+    return t;
+}
+__device__ const SubsetTable kSubsetTable = makeSubsetTable();
 
 __device__ __forceinline__ bool isLeafNode(int node, int n) { return node >= n - 1; }
 
-__device__ void treeletOptimize(int root, int n, int2* child, int* parent, float4* nodeLo, float4* nodeHi,
-    float* subtreeCost, TreeletScratch& s, float costNode)
+// The subsets of a lane in the rounds of sizes 2, 3, 3, 4, 4, 5 (0: none).
+struct LaneSubsets {
+    uint8_t m[6];
+};
+__device__ __forceinline__ LaneSubsets laneSubsets()
 {
     const int lane = threadIdx.x & 31;
-    const int w = threadIdx.x >> 5;
-    __shared__ int sLeaves[kBlock / 32][kTreeletLeaves];
-    __shared__ int sInternals[kBlock / 32][kTreeletLeaves - 1];
-    __shared__ int sLeafCount[kBlock / 32];
+    LaneSubsets l;
+    l.m[0] = lane < 21 ? kSubsetTable.m[lane] : 0;
+    l.m[1] = kSubsetTable.m[21 + lane];
+    l.m[2] = lane < 3 ? kSubsetTable.m[21 + 32 + lane] : 0;
+    l.m[3] = kSubsetTable.m[56 + lane];
+    l.m[4] = lane < 3 ? kSubsetTable.m[56 + 32 + lane] : 0;
+    l.m[5] = lane < 21 ? kSubsetTable.m[91 + lane] : 0;
+    return l;
+}
+
+__device__ void treeletOptimize(int root, int n, int2* child, int* parent, float4* nodeLo, float4* nodeHi,
+    float* subtreeCost, TreeletScratch& s, const LaneSubsets& mine, float costNode)
+{
+    constexpr unsigned int kAll = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
     // --- form the treelet: open the largest-area treelet leaf until 7 leaves ---
-    if (lane == 0) {
-        int leaves[kTreeletLeaves];
-        int internals[kTreeletLeaves - 1];
-        int nl = 2, ni = 1;
-        internals[0] = root;
+    int node = -1, internal = root;
+    bool inner = false;
+    float4 lo = make_float4(0.0f, 0.0f, 0.0f, 0.0f), hi = lo;
+    int2 kids = make_int2(-1, -1);
+    float cost = 0.0f;
+    auto hold = [&](int x) {
+        node = x;
+        inner = !isLeafNode(x, n);
+        lo = __ldcg(&nodeLo[x]);
+        hi = __ldcg(&nodeHi[x]);
+        cost = __ldcg(&subtreeCost[x]);
+        if (inner) {
+            kids = __ldcg(&child[x]);
+        }
+    };
+    {
         const int2 c = __ldcg(&child[root]);
-        leaves[0] = c.x;
-        leaves[1] = c.y;
-        while (nl < kTreeletLeaves) {
-            int best = -1;
-            float bestArea = -1.0f;
-            for (int k = 0; k < nl; ++k) {
-                if (!isLeafNode(leaves[k], n)) {
-                    const float a = __ldcg(&nodeHi[leaves[k]]).w;
-                    if (a > bestArea) {
-                        bestArea = a;
-                        best = k;
-                    }
-                }
-            }
-            if (best < 0) {
-                break;
-            }
-            const int opened = leaves[best];
-            internals[ni++] = opened;
-            const int2 cc = __ldcg(&child[opened]);
-            leaves[best] = cc.x;
-            leaves[nl++] = cc.y;
+        if (lane < 2) {
+            hold(lane == 0 ? c.x : c.y);
         }
-        for (int k = 0; k < nl; ++k) {
-            sLeaves[w][k] = leaves[k];
-        }
-        for (int k = 0; k < ni; ++k) {
-            sInternals[w][k] = internals[k];
-        }
-        sLeafCount[w] = nl;
     }
-    __syncwarp();
-    const int nl = sLeafCount[w];
+    int nl = 2, ni = 1;
+    while (nl < kTreeletLeaves) {
+        // (areas are not negative: their bits order like the values)
+        const unsigned int key = inner && hi.w > -1.0f ? __float_as_uint(hi.w) + 1u : 0u;
+        const unsigned int top = __reduce_max_sync(kAll, key);
+        if (top == 0u) {
+            break;
+        }
+        const int best = __ffs(__ballot_sync(kAll, key == top)) - 1;
+        const int opened = __shfl_sync(kAll, node, best);
+        const int kx = __shfl_sync(kAll, kids.x, best), ky = __shfl_sync(kAll, kids.y, best);
+        if (lane == ni) {
+            internal = opened;
+        }
+        if (lane == best || lane == nl) {
+            hold(lane == best ? kx : ky);
+        }
+        ++ni;
+        ++nl;
+    }
     if (nl < 3) {
         return;
     }
+    if (lane < nl) {
+        s.leafLo[lane] = lo;
+        s.leafHi[lane] = hi;
+        s.leaf[lane] = node;
+        s.cost[1 << lane] = cost; // a treelet leaf keeps its (already optimised) subtree
+        if (lane < ni) {
+            s.internal[lane] = internal;
+        }
+    }
+    __syncwarp();
     const int subsets = 1 << nl;
-    // --- bounds, triangle counts and areas of every leaf subset ---
-    for (int m = lane + 1; m < subsets; m += 32) {
-        float3 lo = make_float3(FLT_MAX, FLT_MAX, FLT_MAX), hi = make_float3(-FLT_MAX, -FLT_MAX, -FLT_MAX);
-        int tris = 0;
-        for (int k = 0; k < nl; ++k) {
-            if (m & (1 << k)) {
-                const float4 a = __ldcg(&nodeLo[sLeaves[w][k]]), b = __ldcg(&nodeHi[sLeaves[w][k]]);
-                lo = make_float3(fminf(lo.x, a.x), fminf(lo.y, a.y), fminf(lo.z, a.z));
-                hi = make_float3(fmaxf(hi.x, b.x), fmaxf(hi.y, b.y), fmaxf(hi.z, b.z));
-                tris += __float_as_int(a.w);
+    // --- area of every leaf subset: bits 2.. from the lane, bits 0 and 1 in turn ---
+    {
+        float3 bl = make_float3(FLT_MAX, FLT_MAX, FLT_MAX), bh = make_float3(-FLT_MAX, -FLT_MAX, -FLT_MAX);
+        auto join = [&](float3& l, float3& h, int k) {
+            const float4 a = s.leafLo[k], b = s.leafHi[k];
+            l = make_float3(fminf(l.x, a.x), fminf(l.y, a.y), fminf(l.z, a.z));
+            h = make_float3(fmaxf(h.x, b.x), fmaxf(h.y, b.y), fmaxf(h.z, b.z));
+        };
+        for (int k = 2; k < nl; ++k) {
+            if ((lane >> (k - 2)) & 1) {
+                join(bl, bh, k);
             }
         }
-        s.lo[m] = make_float4(lo.x, lo.y, lo.z, __int_as_float(tris));
-        s.hi[m] = make_float4(hi.x, hi.y, hi.z, 0.0f);
-        s.area[m] = boxArea(lo, hi);
-        if (__popc(m) == 1) {
-            // a treelet leaf keeps its (already optimised) subtree
-            s.cost[m] = __ldcg(&subtreeCost[sLeaves[w][__ffs(m) - 1]]);
-            s.split[m] = 0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            float3 l = bl, h = bh;
+            if (j & 1) {
+                join(l, h, 0);
+            }
+            if (j & 2) {
+                join(l, h, 1);
+            }
+            const int m = 4 * lane + j;
+            if (m > 0 && m < subsets) {
+                s.area[m] = boxArea(l, h);
+            }
         }
     }
     __syncwarp();
     // --- SAH-optimal topology by dynamic programming over subsets of growing size ---
-    for (int size = 2; size <= nl; ++size) {
-        for (int m = lane + 1; m < subsets; m += 32) {
-            if (__popc(m) != size) {
-                continue;
-            }
+    // A partition is named by its part with the lowest leaf; of equal costs the
+    // largest such part is taken (parts are tried in falling order).
+    auto settle = [&](int m, float best, int part) {
+        s.cost[m] = costNode * s.area[m] + best;
+        s.split[m] = static_cast<uint8_t>(part);
+    };
+#pragma unroll
+    for (int r = 0; r < 6; ++r) {
+        const int m = mine.m[r];
+        if (m != 0 && m < subsets) {
+            const int low = m & -m, rest = m ^ low;
             float best = FLT_MAX;
-            int bestP = 0;
-            const int low = m & -m;
-            for (int p = (m - 1) & m; p > 0; p = (p - 1) & m) {
-                if ((p & low) == 0) {
-                    continue; // each partition once
-                }
-                const float c = s.cost[p] + s.cost[m ^ p];
+            int part = low;
+            for (int q = (rest - 1) & rest;; q = (q - 1) & rest) {
+                const float c = s.cost[low | q] + s.cost[rest ^ q];
                 if (c < best) {
                     best = c;
-                    bestP = p;
+                    part = low | q;
+                }
+                if (q == 0) {
+                    break;
                 }
             }
-            s.cost[m] = costNode * s.area[m] + best;
-            s.split[m] = static_cast<uint8_t>(bestP);
+            settle(m, best, part);
+        }
+        if (r == 0 || r == 2 || r >= 4) {
+            __syncwarp();
+        }
+    }
+    if (nl >= 6) {
+        // seven subsets of six leaves, 31 partitions each, four lanes to a subset
+        const int m = (kSubsets - 1) ^ (1 << (lane >> 2));
+        const bool on = lane < 28 && m < subsets;
+        const int low = m & -m, rest = m ^ low;
+        float best = FLT_MAX;
+        int at = 64, part = low;
+        if (on) {
+            int q = rest;
+            for (int i = 0; i < 31; ++i) {
+                q = (q - 1) & rest;
+                if ((i & 3) == (lane & 3)) {
+                    const float c = s.cost[low | q] + s.cost[rest ^ q];
+                    if (c < best) {
+                        best = c;
+                        at = i;
+                        part = low | q;
+                    }
+                }
+            }
+        }
+#pragma unroll
+        for (int d = 1; d <= 2; d <<= 1) {
+            const float c = __shfl_xor_sync(kAll, best, d);
+            const int i = __shfl_xor_sync(kAll, at, d), pt = __shfl_xor_sync(kAll, part, d);
+            if (c < best || (c == best && i < at)) {
+                best = c;
+                at = i;
+                part = pt;
+            }
+        }
+        if (on && (lane & 3) == 0) {
+            settle(m, best, part);
+        }
+        __syncwarp();
+    }
+    if (nl == kTreeletLeaves) {
+        // all seven leaves: 63 partitions over the warp
+        constexpr int rest = kSubsets - 2;
+        float best = FLT_MAX;
+        int at = 64;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int i = lane + 32 * h;
+            if (i < 63) {
+                const int q = 2 * (62 - i);
+                const float c = s.cost[1 | q] + s.cost[rest ^ q];
+                if (c < best) {
+                    best = c;
+                    at = i;
+                }
+            }
+        }
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const float c = __shfl_xor_sync(kAll, best, d);
+            const int i = __shfl_xor_sync(kAll, at, d);
+            if (c < best || (c == best && i < at)) {
+                best = c;
+                at = i;
+            }
+        }
+        if (lane == 0) {
+            settle(kSubsets - 1, best, at < 63 ? 1 | (2 * (62 - at)) : 1);
         }
         __syncwarp();
     }
     // --- rewrite the treelet in place, reusing its internal node ids ---
     if (lane == 0) {
-        int stackM[kTreeletLeaves];
-        int stackNode[kTreeletLeaves];
-        int sp = 0;
-        int nextInternal = 1;
-        stackM[sp] = subsets - 1;
-        stackNode[sp] = root;
-        ++sp;
+        int stack[kTreeletLeaves];
+        int sp = 0, next = 1;
+        s.mask[0] = static_cast<uint8_t>(subsets - 1);
+        stack[sp++] = 0;
         while (sp > 0) {
-            --sp;
-            const int m = stackM[sp];
-            const int node = stackNode[sp];
+            const int e = stack[--sp];
+            const int m = s.mask[e];
             const int parts[2] = {static_cast<int>(s.split[m]), m ^ static_cast<int>(s.split[m])};
-            int kids[2];
+#pragma unroll
             for (int h = 0; h < 2; ++h) {
-                if (__popc(parts[h]) == 1) {
-                    kids[h] = sLeaves[w][__ffs(parts[h]) - 1];
+                if ((parts[h] & (parts[h] - 1)) == 0) {
+                    s.kids[e][h] = s.leaf[__ffs(parts[h]) - 1];
                 } else {
-                    kids[h] = sInternals[w][nextInternal++];
-                    stackM[sp] = parts[h];
-                    stackNode[sp] = kids[h];
-                    ++sp;
+                    s.mask[next] = static_cast<uint8_t>(parts[h]);
+                    s.kids[e][h] = s.internal[next];
+                    stack[sp++] = next++;
                 }
-                parent[kids[h]] = node;
             }
-            child[node] = make_int2(kids[0], kids[1]);
-            float4 hi = s.hi[m];
-            hi.w = s.area[m];
-            __stcg(&nodeLo[node], s.lo[m]);
-            __stcg(&nodeHi[node], hi);
-            __stcg(&subtreeCost[node], s.cost[m]);
         }
     }
-    __threadfence();
+    __syncwarp();
+    if (lane < ni) {
+        const int m = s.mask[lane];
+        const int2 k = make_int2(s.kids[lane][0], s.kids[lane][1]);
+        float4 l = make_float4(FLT_MAX, FLT_MAX, FLT_MAX, 0.0f), h = make_float4(-FLT_MAX, -FLT_MAX, -FLT_MAX, s.area[m]);
+        int tris = 0;
+        for (int j = 0; j < nl; ++j) {
+            if ((m >> j) & 1) {
+                const float4 a = s.leafLo[j], b = s.leafHi[j];
+                l = make_float4(fminf(l.x, a.x), fminf(l.y, a.y), fminf(l.z, a.z), 0.0f);
+                h = make_float4(fmaxf(h.x, b.x), fmaxf(h.y, b.y), fmaxf(h.z, b.z), h.w);
+                tris += __float_as_int(a.w);
+            }
+        }
+        l.w = __int_as_float(tris);
+        child[internal] = k;
+        parent[k.x] = internal;
+        parent[k.y] = internal;
+        __stcg(&nodeLo[internal], l);
+        __stcg(&nodeHi[internal], h);
+        __stcg(&subtreeCost[internal], s.cost[m]);
+        __threadfence();
+    }
     __syncwarp();
 }
 
-// One warp per leaf climbs towards the root; the warp that reaches a node
-// second (both subtrees final) optimises the treelet rooted there.
 // Bottom-up pass of the subtrees too small for treelets, one thread per leaf
 // (as the refit): the SAH cost of every subtree with fewer than minLeaves
 // triangles, and the list of the nodes where treelet work starts (at least
@@ -399,33 +565,34 @@ __global__ void k_treelet_leaves(int n, const int2* child, const int* parent, co
 // list and then up the tree: a node is optimised by the second warp to reach it
 // (its first arrival may have come from k_treelet_leaves, for a small child).
 // Every node from the frontier up has at least minLeaves triangles.
-__global__ void k_treelet(int n, int2* child, int* parent, float4* nodeLo, float4* nodeHi, int* visits,
-    float* subtreeCost, float costNode, const int* frontier, const unsigned int* frontierCount)
+#ifndef PT_TREELET_BLOCKS
+#define PT_TREELET_BLOCKS 6
+#endif
+__global__ void __launch_bounds__(kBlock, PT_TREELET_BLOCKS) k_treelet(int n, int2* child, int* parent, float4* nodeLo,
+    float4* nodeHi, int* visits, float* subtreeCost, float costNode, const int* frontier,
+    const unsigned int* frontierCount)
 {
     __shared__ TreeletScratch scratch[kBlock / 32];
     const int lane = threadIdx.x & 31;
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int warps = (gridDim.x * blockDim.x) >> 5;
     TreeletScratch& s = scratch[threadIdx.x >> 5];
+    const LaneSubsets mine = laneSubsets();
     const int count = static_cast<int>(*frontierCount);
     for (int f = warp; f < count; f += warps) {
         int p = frontier[f];
         for (;;) {
-            treeletOptimize(p, n, child, parent, nodeLo, nodeHi, subtreeCost, s, costNode);
-            __threadfence();
-            p = __shfl_sync(0xffffffffu, lane == 0 ? __ldcg(&parent[p]) : 0, 0);
-            if (p < 0) {
-                break;
-            }
+            treeletOptimize(p, n, child, parent, nodeLo, nodeHi, subtreeCost, s, mine, costNode);
             int arrived = 0;
             if (lane == 0) {
-                arrived = atomicAdd(&visits[p], 1);
+                p = __ldcg(&parent[p]);
+                arrived = p >= 0 ? atomicAdd(&visits[p], 1) : 0;
+                __threadfence();
             }
-            arrived = __shfl_sync(0xffffffffu, arrived, 0);
-            if (arrived == 0) {
-                break;
+            p = __shfl_sync(0xffffffffu, p, 0);
+            if (__shfl_sync(0xffffffffu, arrived, 0) == 0) {
+                break; // the sibling's warp goes on, or this was the root
             }
-            __threadfence();
         }
     }
 }
@@ -449,14 +616,14 @@ static cudaError_t runTreelets(int N, int2* child, int* parent, float4* nodeLo, 
         int dev = 0, sms = 1;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        k_treelet<<<sms * 4, kBlock, 0, stream>>>(N, child, parent, nodeLo, nodeHi, visits, subCost, opt.costNode,
+        k_treelet<<<sms * PT_TREELET_BLOCKS, kBlock, 0, stream>>>(N, child, parent, nodeLo, nodeHi, visits, subCost, opt.costNode,
             frontier, frontierCount);
     }
     return cudaGetLastError();
 }
 
-// (7) Collapse to 8-wide compressed nodes. One thread per task (binary node ->
-// compressed node slot). Emits the next level's tasks.
+// (7) Collapse to 8-wide compressed nodes, level by level: a task is a binary
+// node and the slot of its compressed node; a level emits the next one's tasks.
 struct CollapseArgs {
     int n;
     const int2* child;
@@ -466,7 +633,7 @@ struct CollapseArgs {
     const float* pos;
     CwNode* cw;
     TriVerts* tris;
-    unsigned int* counters; // [0] next node, [1] next triangle
+    unsigned int* counters; // [0] next node, [1] next triangle, [2], [3] tasks of even and odd levels
     int maxLeafSize;
 };
 
@@ -485,146 +652,196 @@ __device__ __forceinline__ int quantExp(double extent)
     return max(e, -126);
 }
 
-__global__ void k_collapse(CollapseArgs a, const int2* __restrict__ tasks, int taskCount, int2* __restrict__ nextTasks,
-    unsigned int* __restrict__ nextCount)
+// Eight lanes per task, one per child.  Bound by latency: a level has few tasks
+// at the top, and one thread per task walked its eight children one after the
+// other (boxes, 64-entry cost table, quantisation in double, triangle records):
+// 50 - 160 us per level, 11 levels for 972k triangles; now 330 us in all
+// against 916.  The task count of a level stays on the device, so that the host
+// asks only once per kCollapseAhead levels whether there are more.
+constexpr int kCollapseThreads = 128;
+constexpr int kCollapseAhead = 4;
+
+__global__ void __launch_bounds__(kCollapseThreads) k_collapse(CollapseArgs a, const int2* __restrict__ tasks,
+    int2* __restrict__ nextTasks, int level)
 {
-    for (int ti = blockIdx.x * blockDim.x + threadIdx.x; ti < taskCount; ti += gridDim.x * blockDim.x) {
-        const int bnode = tasks[ti].x;
-        const int cwIndex = tasks[ti].y;
-        int cand[8];
+    constexpr unsigned int kAll = 0xffffffffu;
+    __shared__ uint4 sNode[kCollapseThreads / 8][5];
+    const int taskCount = static_cast<int>(a.counters[2 + (level & 1)]);
+    unsigned int* nextCount = &a.counters[2 + ((level & 1) ^ 1)];
+    const int lane = threadIdx.x & 31, k = lane & 7, first = lane & 24;
+    const int group = (blockIdx.x * blockDim.x + threadIdx.x) >> 3, groups = (gridDim.x * blockDim.x) >> 3;
+    uint4* words = sNode[threadIdx.x >> 3];
+    uint8_t* bytes = reinterpret_cast<uint8_t*>(words);
+    // (a warp's four groups loop together)
+    for (int t0 = group - (lane >> 3); t0 < taskCount; t0 += groups) {
+        const int ti = t0 + (lane >> 3);
+        const bool valid = ti < taskCount;
+        const int2 task = valid ? tasks[ti] : make_int2(0, 0);
+        const int bnode = task.x;
+        // --- children: open the largest-area candidate until 8 slots are used, first
+        // those that are too big for a leaf, then the remaining internal ones ---
+        int cand = -1, count = 0;
+        bool inner = false;
+        float4 cl = make_float4(0.0f, 0.0f, 0.0f, 0.0f), ch = cl;
+        int2 kids = make_int2(-1, -1);
+        auto hold = [&](int x) {
+            cand = x;
+            inner = !isLeafNode(x, a.n);
+            cl = a.nodeLo[x];
+            ch = a.nodeHi[x];
+            count = __float_as_int(cl.w);
+            if (inner) {
+                kids = a.child[x];
+            }
+        };
+        float4 nl4 = cl, nh4 = cl;
         int nc = 0;
-        if (isLeafNode(bnode, a.n)) {
-            cand[nc++] = bnode;
-        } else {
-            const int2 c = a.child[bnode];
-            cand[nc++] = c.x;
-            cand[nc++] = c.y;
-        }
-        // Open the largest-area candidate until 8 slots are used: first those
-        // that are too big for a leaf, then the remaining internal ones.
-        while (nc < 8) {
-            int best = -1;
-            float bestArea = -1.0f;
-            bool bestBig = false;
-            for (int k = 0; k < nc; ++k) {
-                if (isLeafNode(cand[k], a.n)) {
-                    continue;
+        if (valid) {
+            nl4 = a.nodeLo[bnode];
+            nh4 = a.nodeHi[bnode];
+            if (isLeafNode(bnode, a.n)) {
+                nc = 1;
+                if (k == 0) {
+                    hold(bnode);
                 }
-                const bool big = __float_as_int(a.nodeLo[cand[k]].w) > a.maxLeafSize;
-                const float ar = a.nodeHi[cand[k]].w;
-                if ((big && !bestBig) || (big == bestBig && ar > bestArea)) {
-                    best = k;
-                    bestArea = ar;
-                    bestBig = big;
+            } else {
+                const int2 c = a.child[bnode];
+                nc = 2;
+                if (k < 2) {
+                    hold(k == 0 ? c.x : c.y);
                 }
             }
-            if (best < 0) {
-                break;
-            }
-            const int2 c = a.child[cand[best]];
-            cand[best] = c.x;
-            cand[nc++] = c.y;
         }
-        // Node bounds.
-        const float4 nl4 = a.nodeLo[bnode], nh4 = a.nodeHi[bnode];
+        for (int r = 0; r < 6; ++r) {
+            // (areas are not negative: their bits order like the values)
+            unsigned int key = 0u;
+            if (inner && nc < 8 && ch.w > -1.0f) {
+                key = (__float_as_uint(ch.w) + 1u) | (count > a.maxLeafSize ? 0x80000000u : 0u);
+            }
+            unsigned int top = key;
+#pragma unroll
+            for (int d = 1; d < 8; d <<= 1) {
+                top = max(top, __shfl_xor_sync(kAll, top, d));
+            }
+            const unsigned int at = __ballot_sync(kAll, key == top) >> first;
+            const int best = __ffs(at & 0xffu) - 1;
+            const int kx = __shfl_sync(kAll, kids.x, first + best), ky = __shfl_sync(kAll, kids.y, first + best);
+            if (top != 0u) {
+                if (k == best || k == nc) {
+                    hold(k == best ? kx : ky);
+                }
+                ++nc;
+            }
+        }
+        // --- node bounds ---
         const float3 lo = make_float3(nl4.x, nl4.y, nl4.z);
         const float3 hi = make_float3(nh4.x, nh4.y, nh4.z);
-        const int ex = quantExp(static_cast<double>(hi.x) - lo.x), ey = quantExp(static_cast<double>(hi.y) - lo.y),
-                  ez = quantExp(static_cast<double>(hi.z) - lo.z);
-        const double sx = ldexp(1.0, ex), sy = ldexp(1.0, ey), sz = ldexp(1.0, ez);
-        // Octant-ordered slot assignment: slot s receives the child that is nearest
-        // for rays whose direction signs are s (bit 2 = -x, bit 1 = -y, bit 0 = -z).
+        const float extLo = k == 0 ? lo.x : (k == 1 ? lo.y : lo.z), extHi = k == 0 ? hi.x : (k == 1 ? hi.y : hi.z);
+        const int own = valid && k < 3 ? quantExp(static_cast<double>(extHi) - extLo) : 0;
+        const int ex = __shfl_sync(kAll, own, first), ey = __shfl_sync(kAll, own, first + 1),
+                  ez = __shfl_sync(kAll, own, first + 2);
+        // --- octant-ordered slot assignment: slot s receives the child that is nearest
+        // for rays whose direction signs are s (bit 2 = -x, bit 1 = -y, bit 0 = -z) ---
         const float3 nc3 = make_float3((lo.x + hi.x) * 0.5f, (lo.y + hi.y) * 0.5f, (lo.z + hi.z) * 0.5f);
-        float cost[8][8];
-        for (int k = 0; k < nc; ++k) {
-            const float4 cl = a.nodeLo[cand[k]], ch = a.nodeHi[cand[k]];
-            const float3 d = make_float3((cl.x + ch.x) * 0.5f - nc3.x, (cl.y + ch.y) * 0.5f - nc3.y,
-                (cl.z + ch.z) * 0.5f - nc3.z);
-            for (int s = 0; s < 8; ++s) {
-                const float dx = (s & 4) ? -d.x : d.x;
-                const float dy = (s & 2) ? -d.y : d.y;
-                const float dz = (s & 1) ? -d.z : d.z;
-                cost[k][s] = dx + dy + dz;
-            }
-        }
-        int slotOf[8];
-        int bySlot[8];
-        for (int s = 0; s < 8; ++s) {
-            bySlot[s] = -1;
-        }
-        for (int k = 0; k < nc; ++k) {
-            slotOf[k] = -1;
-        }
-        for (int round = 0; round < nc; ++round) {
+        const float3 d3 = make_float3((cl.x + ch.x) * 0.5f - nc3.x, (cl.y + ch.y) * 0.5f - nc3.y,
+            (cl.z + ch.z) * 0.5f - nc3.z);
+        int slot = -1;
+        unsigned int taken = 0u;
+        for (int round = 0; round < 8; ++round) {
+            // the cheapest free (child, slot) pair; of equal ones the first child's first slot
             float best = FLT_MAX;
-            int bk = -1, bs = -1;
-            for (int k = 0; k < nc; ++k) {
-                if (slotOf[k] >= 0) {
-                    continue;
-                }
+            int bs = -1;
+            if (slot < 0 && k < nc) {
+#pragma unroll
                 for (int s = 0; s < 8; ++s) {
-                    if (bySlot[s] >= 0) {
-                        continue;
-                    }
-                    if (cost[k][s] < best || bk < 0) {
-                        best = cost[k][s];
-                        bk = k;
+                    const float dx = (s & 4) ? -d3.x : d3.x;
+                    const float dy = (s & 2) ? -d3.y : d3.y;
+                    const float dz = (s & 1) ? -d3.z : d3.z;
+                    const float c = dx + dy + dz;
+                    if (((taken >> s) & 1u) == 0u && (c < best || bs < 0)) {
+                        best = c;
                         bs = s;
                     }
                 }
             }
-            slotOf[bk] = bs;
-            bySlot[bs] = bk;
-        }
-        // Count internal children and leaf triangles.
-        int internals = 0, triTotal = 0;
-        for (int k = 0; k < nc; ++k) {
-            const int cnt = __float_as_int(a.nodeLo[cand[k]].w);
-            if (cnt > a.maxLeafSize) {
-                ++internals;
-            } else {
-                triTotal += cnt;
+            // (+ 0: -0 counts as 0; the key orders like the cost and is not 0)
+            const unsigned int key = bs < 0 ? 0xffffffffu : min(floatToOrdered(best + 0.0f), 0xfffffffeu);
+            unsigned int low = key;
+#pragma unroll
+            for (int d = 1; d < 8; d <<= 1) {
+                low = min(low, __shfl_xor_sync(kAll, low, d));
+            }
+            const unsigned int at = __ballot_sync(kAll, key == low) >> first;
+            const int win = __ffs(at & 0xffu) - 1;
+            const int ws = __shfl_sync(kAll, bs, first + win);
+            if (low != 0xffffffffu) {
+                if (k == win) {
+                    slot = ws;
+                }
+                taken |= 1u << ws;
             }
         }
-        const unsigned int childBase = internals ? atomicAdd(&a.counters[0], static_cast<unsigned>(internals)) : 0u;
-        const unsigned int triBase = triTotal ? atomicAdd(&a.counters[1], static_cast<unsigned>(triTotal)) : 0u;
-        unsigned int taskBase = internals ? atomicAdd(nextCount, static_cast<unsigned>(internals)) : 0u;
-
-        uint8_t meta[8], qlo[3][8], qhi[3][8];
-        unsigned int imask = 0;
-        int rank = 0, triOff = 0;
-        for (int s = 0; s < 8; ++s) {
-            meta[s] = 0;
-            qlo[0][s] = qlo[1][s] = qlo[2][s] = 0;
-            qhi[0][s] = qhi[1][s] = qhi[2][s] = 0;
-            const int k = bySlot[s];
-            if (k < 0) {
-                continue;
+        // --- internal children and leaf triangles, in slot order ---
+        const bool used = valid && slot >= 0;
+        const bool internal = used && count > a.maxLeafSize;
+        unsigned int imask = internal ? 1u << slot : 0u;
+        unsigned int counts = used && !internal ? static_cast<unsigned int>(count) << (2 * slot) : 0u; // two bits per slot
+#pragma unroll
+        for (int d = 1; d < 8; d <<= 1) {
+            imask |= __shfl_xor_sync(kAll, imask, d);
+            counts |= __shfl_xor_sync(kAll, counts, d);
+        }
+        auto triangles = [](unsigned int c) { return __popc(c & 0x5555u) + 2 * __popc(c & 0xAAAAu); };
+        const unsigned int internals = __popc(imask), triTotal = triangles(counts);
+        unsigned int childBase = 0u, triBase = 0u, taskBase = 0u;
+        if (k == 0 && internals != 0u) {
+            childBase = atomicAdd(&a.counters[0], internals);
+            taskBase = atomicAdd(nextCount, internals);
+        }
+        if (k == 0 && triTotal != 0u) {
+            triBase = atomicAdd(&a.counters[1], triTotal);
+        }
+        childBase = __shfl_sync(kAll, childBase, first);
+        taskBase = __shfl_sync(kAll, taskBase, first);
+        triBase = __shfl_sync(kAll, triBase, first);
+        // --- the compressed node, put together in shared memory ---
+        if (k < 5) {
+            uint4 w = make_uint4(0u, 0u, 0u, 0u);
+            if (k == 0) {
+                w = make_uint4(__float_as_uint(lo.x), __float_as_uint(lo.y), __float_as_uint(lo.z),
+                    static_cast<unsigned>(ex + 127) | (static_cast<unsigned>(ey + 127) << 8) |
+                        (static_cast<unsigned>(ez + 127) << 16) | (imask << 24));
+            } else if (k == 1) {
+                w.x = childBase;
+                w.y = triBase;
             }
-            const int c = cand[k];
-            const float4 cl = a.nodeLo[c], ch = a.nodeHi[c];
+            words[k] = w;
+        }
+        __syncwarp();
+        if (used) {
             const float clv[3] = {cl.x, cl.y, cl.z};
             const float chv[3] = {ch.x, ch.y, ch.z};
             const float pv[3] = {lo.x, lo.y, lo.z};
-            const double sv[3] = {sx, sy, sz};
+            const int ev[3] = {ex, ey, ez};
+#pragma unroll
             for (int ax = 0; ax < 3; ++ax) {
-                const double ql = floor((static_cast<double>(clv[ax]) - static_cast<double>(pv[ax])) / sv[ax]);
-                const double qh = ceil((static_cast<double>(chv[ax]) - static_cast<double>(pv[ax])) / sv[ax]);
-                qlo[ax][s] = static_cast<uint8_t>(fmin(fmax(ql, 0.0), 255.0));
-                qhi[ax][s] = static_cast<uint8_t>(fmin(fmax(qh, 0.0), 255.0));
+                const double inv = ldexp(1.0, -ev[ax]); // (a power of two: the product is the exact quotient)
+                const double ql = floor((static_cast<double>(clv[ax]) - static_cast<double>(pv[ax])) * inv);
+                const double qh = ceil((static_cast<double>(chv[ax]) - static_cast<double>(pv[ax])) * inv);
+                bytes[32 + 8 * ax + slot] = static_cast<uint8_t>(fmin(fmax(ql, 0.0), 255.0));
+                bytes[56 + 8 * ax + slot] = static_cast<uint8_t>(fmin(fmax(qh, 0.0), 255.0));
             }
-            const int cnt = __float_as_int(cl.w);
-            if (cnt > a.maxLeafSize) {
-                meta[s] = static_cast<uint8_t>(0x20 | (24 + s));
-                imask |= 1u << s;
-                nextTasks[taskBase + rank] = make_int2(c, static_cast<int>(childBase) + rank);
-                ++rank;
+            if (internal) {
+                bytes[24 + slot] = static_cast<uint8_t>(0x20 | (24 + slot));
+                const int rank = __popc(imask & ((1u << slot) - 1u));
+                nextTasks[taskBase + rank] = make_int2(cand, static_cast<int>(childBase) + rank);
             } else {
-                meta[s] = static_cast<uint8_t>((((1 << cnt) - 1) << 5) | triOff);
+                unsigned int triOff = triangles(counts & ((1u << (2 * slot)) - 1u));
+                bytes[24 + slot] = static_cast<uint8_t>((((1 << count) - 1) << 5) | triOff);
                 // gather the subtree's triangles (at most maxLeafSize leaves)
                 int st[8];
                 int sp = 0;
-                st[sp++] = c;
+                st[sp++] = cand;
                 while (sp > 0) {
                     const int x = st[--sp];
                     if (isLeafNode(x, a.n)) {
@@ -645,19 +862,11 @@ __global__ void k_collapse(CollapseArgs a, const int2* __restrict__ tasks, int t
                 }
             }
         }
-        CwNode node;
-        node.w[0] = make_uint4(__float_as_uint(lo.x), __float_as_uint(lo.y), __float_as_uint(lo.z),
-            static_cast<unsigned>(ex + 127) | (static_cast<unsigned>(ey + 127) << 8) |
-                (static_cast<unsigned>(ez + 127) << 16) | (imask << 24));
-        auto pack4 = [](const uint8_t* b) {
-            return static_cast<unsigned>(b[0]) | (static_cast<unsigned>(b[1]) << 8) |
-                (static_cast<unsigned>(b[2]) << 16) | (static_cast<unsigned>(b[3]) << 24);
-        };
-        node.w[1] = make_uint4(childBase, triBase, pack4(meta), pack4(meta + 4));
-        node.w[2] = make_uint4(pack4(qlo[0]), pack4(qlo[0] + 4), pack4(qlo[1]), pack4(qlo[1] + 4));
-        node.w[3] = make_uint4(pack4(qlo[2]), pack4(qlo[2] + 4), pack4(qhi[0]), pack4(qhi[0] + 4));
-        node.w[4] = make_uint4(pack4(qhi[1]), pack4(qhi[1] + 4), pack4(qhi[2]), pack4(qhi[2] + 4));
-        a.cw[cwIndex] = node;
+        __syncwarp();
+        if (valid && k < 5) {
+            a.cw[task.y].w[k] = words[k];
+        }
+        __syncwarp();
     }
 }
 
@@ -684,11 +893,31 @@ inline int gridFor(long long n, int block = kBlock)
         }                                                                                                         \
     } while (0)
 
+// All levels of the collapse, from the root task in taskA and counters[2] = 1.
+static int runCollapse(const CollapseArgs& ca, int2* taskA, int2* taskB, cudaStream_t stream, char* err, size_t errLen)
+{
+    constexpr int kBlocks = 148 * 8;
+    const int blocks = std::min<long long>(kBlocks, (static_cast<long long>(ca.n) + kCollapseThreads / 8 - 1) / (kCollapseThreads / 8));
+    for (int level = 0; level < 256; ++level) {
+        PT_TRY(cudaMemsetAsync(ca.counters + 2 + ((level & 1) ^ 1), 0, sizeof(unsigned int), stream));
+        k_collapse<<<blocks, kCollapseThreads, 0, stream>>>(ca, (level & 1) ? taskB : taskA, (level & 1) ? taskA : taskB, level);
+        if (level % kCollapseAhead == kCollapseAhead - 1) {
+            unsigned int next = 0;
+            PT_TRY(cudaMemcpyAsync(&next, ca.counters + 2 + ((level & 1) ^ 1), sizeof(unsigned int), cudaMemcpyDeviceToHost, stream));
+            PT_TRY(cudaStreamSynchronize(stream));
+            if (next == 0) {
+                return PT_OK;
+            }
+        }
+    }
+    std::snprintf(err, errLen, "BVH collapse did not terminate");
+    return PT_ERR_INTERNAL;
+}
+
 int buildBvh(const float* dPositions, uint32_t n, BvhBuffers& out, cudaStream_t stream, const BvhBuildOptions& opt,
     char* err, size_t errLen)
 {
     out.nodeCount = out.triCount = 0;
-    out.levels = 0;
     if (n == 0) {
         return PT_OK;
     }
@@ -716,7 +945,7 @@ int buildBvh(const float* dPositions, uint32_t n, BvhBuffers& out, cudaStream_t 
     // bounds sentinel: min slots get 0xFFFFFFFF, max slots 0
     const unsigned int init[8] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0u, 0u, 0u, 0u, 0u};
     PT_TRY(cudaMemcpyAsync(cbounds, init, sizeof(init), cudaMemcpyHostToDevice, stream));
-    k_prepare<<<gridFor(n), kBlock, 0, stream>>>(dPositions, n, triLo, triHi, cbounds);
+    k_prepare<<<std::min(gridFor(n), 148 * 8), kBlock, 0, stream>>>(dPositions, n, triLo, triHi, cbounds);
     k_morton<<<gridFor(n), kBlock, 0, stream>>>(triLo, triHi, n, cbounds, keys, vals);
     const size_t tempBytes = radixSortTempBytes(n);
     void* temp = ar.getBytes(13, tempBytes);
@@ -757,36 +986,22 @@ int buildBvh(const float* dPositions, uint32_t n, BvhBuffers& out, cudaStream_t 
         std::snprintf(err, errLen, "collapse scratch allocation failed");
         return PT_ERR_OUT_OF_MEMORY;
     }
-    // counters: [0] next node (root = 0 already taken), [1] next triangle, [2] next task count
-    const unsigned int cinit[4] = {1u, 0u, 0u, 0u};
+    // counters: [0] next node (root = 0 already taken), [1] next triangle, [2] tasks of level 0
+    const unsigned int cinit[4] = {1u, 0u, 1u, 0u};
     PT_TRY(cudaMemcpyAsync(counters, cinit, sizeof(cinit), cudaMemcpyHostToDevice, stream));
     const int rootBin = N > 1 ? 0 : 0; // internal root 0, or the single leaf node 0 (= n - 1) when n == 1
     const int2 rootTask = make_int2(N > 1 ? rootBin : 0, 0);
     PT_TRY(cudaMemcpyAsync(taskA, &rootTask, sizeof(int2), cudaMemcpyHostToDevice, stream));
     CollapseArgs ca{N, child, nodeLo, nodeHi, valsSorted, dPositions, out.nodes, out.tris, counters, opt.maxLeafSize};
-    int taskCount = 1;
-    int levels = 0;
-    while (taskCount > 0) {
-        PT_TRY(cudaMemsetAsync(counters + 2, 0, sizeof(unsigned int), stream));
-        k_collapse<<<gridFor(taskCount, 64), 64, 0, stream>>>(ca, taskA, taskCount, taskB, counters + 2);
-        unsigned int next = 0;
-        PT_TRY(cudaMemcpyAsync(&next, counters + 2, sizeof(unsigned int), cudaMemcpyDeviceToHost, stream));
-        PT_TRY(cudaStreamSynchronize(stream));
-        taskCount = static_cast<int>(next);
-        int2* t = taskA;
-        taskA = taskB;
-        taskB = t;
-        if (++levels > 256) {
-            std::snprintf(err, errLen, "BVH collapse did not terminate");
-            return PT_ERR_INTERNAL;
-        }
+    const int st = runCollapse(ca, taskA, taskB, stream, err, errLen);
+    if (st != PT_OK) {
+        return st;
     }
     unsigned int finalCounts[2] = {0, 0};
     PT_TRY(cudaMemcpyAsync(finalCounts, counters, sizeof(finalCounts), cudaMemcpyDeviceToHost, stream));
     PT_TRY(cudaStreamSynchronize(stream));
     out.nodeCount = finalCounts[0];
     out.triCount = finalCounts[1];
-    out.levels = levels;
     if (out.triCount != n) {
         std::snprintf(err, errLen, "BVH collapse placed %u of %u triangles", out.triCount, n);
         return PT_ERR_INTERNAL;
@@ -815,7 +1030,7 @@ int buildBvhInto(const float* dPositions, uint32_t n, const BvhScratch& sc, CwNo
     const int nodesBin = 2 * N - 1;
     const unsigned int init[8] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0u, 0u, 0u, 0u, 0u};
     PT_TRY(cudaMemcpyAsync(sc.cbounds, init, sizeof(init), cudaMemcpyHostToDevice, stream));
-    k_prepare<<<gridFor(n), kBlock, 0, stream>>>(dPositions, n, sc.triLo, sc.triHi, sc.cbounds);
+    k_prepare<<<std::min(gridFor(n), 148 * 8), kBlock, 0, stream>>>(dPositions, n, sc.triLo, sc.triHi, sc.cbounds);
     k_morton<<<gridFor(n), kBlock, 0, stream>>>(sc.triLo, sc.triHi, n, sc.cbounds, sc.keys, sc.vals);
     const size_t tempBytes = radixSortTempBytes(n);
     if (tempBytes > sc.sortTempBytes) {
@@ -835,30 +1050,15 @@ int buildBvhInto(const float* dPositions, uint32_t n, const BvhScratch& sc, CwNo
             sc.frontierCount, opt, stream));
     }
     PT_TRY(cudaGetLastError());
-    const unsigned int cinit[4] = {1u, 0u, 0u, 0u};
+    const unsigned int cinit[4] = {1u, 0u, 1u, 0u};
     PT_TRY(cudaMemcpyAsync(sc.counters, cinit, sizeof(cinit), cudaMemcpyHostToDevice, stream));
     const int2 rootTask = make_int2(0, 0);
     PT_TRY(cudaMemcpyAsync(sc.taskA, &rootTask, sizeof(int2), cudaMemcpyHostToDevice, stream));
     CollapseArgs ca{N, sc.child, sc.nodeLo, sc.nodeHi, sc.valsSorted, dPositions, outNodes, outTris, sc.counters,
         opt.maxLeafSize};
-    int2* taskA = sc.taskA;
-    int2* taskB = sc.taskB;
-    int taskCount = 1;
-    int levels = 0;
-    while (taskCount > 0) {
-        PT_TRY(cudaMemsetAsync(sc.counters + 2, 0, sizeof(unsigned int), stream));
-        k_collapse<<<gridFor(taskCount, 64), 64, 0, stream>>>(ca, taskA, taskCount, taskB, sc.counters + 2);
-        unsigned int next = 0;
-        PT_TRY(cudaMemcpyAsync(&next, sc.counters + 2, sizeof(unsigned int), cudaMemcpyDeviceToHost, stream));
-        PT_TRY(cudaStreamSynchronize(stream));
-        taskCount = static_cast<int>(next);
-        int2* t = taskA;
-        taskA = taskB;
-        taskB = t;
-        if (++levels > 256) {
-            std::snprintf(err, errLen, "BVH collapse did not terminate");
-            return PT_ERR_INTERNAL;
-        }
+    const int st = runCollapse(ca, sc.taskA, sc.taskB, stream, err, errLen);
+    if (st != PT_OK) {
+        return st;
     }
     unsigned int finalCounts[2] = {0, 0};
     PT_TRY(cudaMemcpyAsync(finalCounts, sc.counters, sizeof(finalCounts), cudaMemcpyDeviceToHost, stream));

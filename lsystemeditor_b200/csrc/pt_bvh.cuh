@@ -82,7 +82,6 @@ struct BvhBuffers {
     TriVerts* tris = nullptr;
     uint32_t nodeCount = 0;
     uint32_t triCount = 0;
-    int levels = 0;
     size_t nodeCapacity = 0; // allocated entries, kept across builds
     size_t triCapacity = 0;
     DeviceArena scratch;
@@ -130,7 +129,6 @@ struct BvhBuffers {
         tris = nullptr;
         nodeCapacity = triCapacity = 0;
         nodeCount = triCount = 0;
-        levels = 0;
     }
 };
 

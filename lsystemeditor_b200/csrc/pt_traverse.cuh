@@ -49,7 +49,7 @@ namespace pt {
 #endif
 #ifndef PT_TRACE_CHUNK
 // (smaller: the atomics, on one address, cost more; larger: warps end a launch
-// apart; 1M camera rays 362 us at 128, 240 at 32; 16.7M 2.22 and 2.17 ms)
+// apart; 1M camera rays 362 us at 128, 223 at 32)
 #define PT_TRACE_CHUNK 32
 #endif
 constexpr int kTraceThreads = 128;
