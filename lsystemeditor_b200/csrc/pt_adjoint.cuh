@@ -17,9 +17,20 @@ int adjointBlocksPerSm();
 // null to recompute it with a first replay of the path.
 void launchAdjoint(const LaunchCtx* ctx, const float* dImage, int channels, int spp, int pixels, int materialCount,
     float* grad, const float4* record, int grid, cudaStream_t s);
-// Preview pass of a width x height image (one centred sample per pixel, no
-// accumulation) into out, with the path-replay kernel.
-void launchPreview(const LaunchCtx* ctx, int width, int height, uint32_t globalSeed, int maxDepth, float4* out,
-    int grid, bool inst, cudaStream_t s);
+// Preview passes (one centred sample per pixel, no accumulation) of `levels`
+// consecutive levels with the path-replay kernel; level i draws with global
+// seed i + 1.
+constexpr int kPreviewsPerLaunch = 16;
+struct PreviewArgs {
+    int width[kPreviewsPerLaunch];
+    int height[kPreviewsPerLaunch];
+    size_t offset[kPreviewsPerLaunch]; // first pixel of a level in out
+    int first;                         // level in entry 0
+    int levels;
+    int maxDepth;
+    long long total; // pixels
+    float4* out;
+};
+void launchPreview(const LaunchCtx* ctx, const PreviewArgs& a, int smCount, bool inst, cudaStream_t s);
 
 } // namespace pt

@@ -888,16 +888,22 @@ int renderPreviews(pt_renderer* r)
     if (c == nullptr) {
         return fail(r, PT_ERR_CUDA, "launch context upload failed");
     }
-    const int grid = r->smCount * adjointBlocksPerSm();
-    for (int lv = r->previewDone + 1; lv < r->previewLevels; ++lv) {
-        int w, h, ds;
-        previewDims(r->width, r->height, r->previewLevels, lv, w, h, ds);
-        launchPreview(c, w, h, static_cast<uint32_t>(lv + 1), kPreviewDepth,
-            r->previewBuf.p + previewOffset(r->width, r->height, r->previewLevels, lv), grid,
-            r->scenes[0].instanceCount > 0, r->stream);
+    while (r->previewDone + 1 < r->previewLevels) {
+        PreviewArgs a{};
+        a.first = r->previewDone + 1;
+        a.levels = std::min(r->previewLevels - a.first, kPreviewsPerLaunch);
+        a.maxDepth = kPreviewDepth;
+        a.out = r->previewBuf.p;
+        for (int k = 0; k < a.levels; ++k) {
+            int ds;
+            previewDims(r->width, r->height, r->previewLevels, a.first + k, a.width[k], a.height[k], ds);
+            a.offset[k] = previewOffset(r->width, r->height, r->previewLevels, a.first + k);
+            a.total += static_cast<long long>(a.width[k]) * a.height[k];
+        }
+        launchPreview(c, a, r->smCount, r->scenes[0].instanceCount > 0, r->stream);
         PT_CHECK(r, cudaGetLastError());
         r->launches += 1;
-        r->previewDone = lv;
+        r->previewDone = a.first + a.levels - 1;
     }
     return PT_OK;
 }
