@@ -218,7 +218,7 @@ __device__ float3 replayPath(const LaunchCtx& c, const PathStart& ps, float3 del
         const bool hit =
             traceRay<false, false, Inst>(S, ro, xnormalize(rd), tMin, kRayTMax, h, nullptr, nullptr, sstack, kAdjointBlock);
         if (!hit) {
-            // k_shade_miss: the pending next-event terms are already in L
+            // shadeMiss: the pending next-event terms are already in L
             if (depth == 0) {
                 L = envEval(c.env, c.params, rd);
             } else {

@@ -241,7 +241,6 @@ struct pt_renderer {
     int gridShadowLane = 0;          // grid of the per-lane shadow kernel
     int gridExtendLaneInst = 0;      // grids of the per-lane kernels of instanced scenes
     int gridShadowLaneInst = 0;
-    int gridShadeMiss = 0;           // grid of the miss shader (its own occupancy)
     bool extendLane = false;         // per-lane ray replacement in this render's closest-hit stage
     int extendMode = PT_EXTEND_MODE_AUTO;
     // CUDA graphs of four bounce iterations (the first block of a batch, later
@@ -546,7 +545,6 @@ int resetAccum(pt_renderer* r)
 }
 
 enum Stage { kGenerate = 0, kExtend, kShade, kShadow, kFinalize, kAccumulate, kCompact, kStageCount };
-// (the miss-shading kernel is accounted to kShade)
 
 // Stage timing: a pair of events around each launch when profiling is on.
 struct StageTimer {
@@ -1265,7 +1263,6 @@ bool ensureBounceGraphs(pt_renderer* r, const LaunchCtx* c, bool inst, int nw)
             (static_cast<unsigned long long>(r->extendLane ? 1 : 0) << 8) |
             (static_cast<unsigned long long>(r->gridExtendLane) << 9) |
             (static_cast<unsigned long long>(r->gridShadowLane) << 22) |
-            (static_cast<unsigned long long>(r->gridShadeMiss) << 36) |
             (static_cast<unsigned long long>(r->scenes.size() > 1 ? 1 : 0) << 62),
         reinterpret_cast<unsigned long long>(r->stream)};
     if (r->bounceGraph[0] != nullptr && std::equal(key, key + 6, r->bounceKey)) {
@@ -1286,13 +1283,9 @@ bool ensureBounceGraphs(pt_renderer* r, const LaunchCtx* c, bool inst, int nw)
         int sel = 0;
         for (int it = 0; it < 4; ++it) {
             launchExtend(c, sel, g == 0 && it == 0, it, extendGrid(r, false, inst), false, inst, r->extendLane, r->scenes.size() > 1, s);
-            launchShadeMiss(c, it, sel, r->gridShadeMiss, nw, s);
             launchShade(c, sel, it, shadeGrid(r, nw), nw, s);
             launchShadow(c, it, shadowGrid(r, false, inst), false, inst, r->extendLane, r->scenes.size() > 1, s);
-            launchFinalize(c, sel, r->gridShadow, nw, s);
-            if (slotOrdered(r)) {
-                launchNextQueue(c, sel, r->gridShadow, s);
-            }
+            launchFinalize(c, sel, r->gridShadow, nw, slotOrdered(r), s);
             sel ^= 1;
         }
         cudaGraph_t graph = nullptr;
@@ -1352,7 +1345,6 @@ int pt_create(pt_renderer** out, int device)
     r->gridShadowLane = r->smCount * shadowLaneOccupancy();
     r->gridExtendLaneInst = r->smCount * extendLaneInstOccupancy();
     r->gridShadowLaneInst = r->smCount * shadowLaneInstOccupancy();
-    r->gridShadeMiss = r->smCount * shadeMissOccupancy();
     *out = r;
     return PT_OK;
 }
@@ -1725,7 +1717,7 @@ int pt_render(pt_renderer* r, int waves)
                     return fail(r, PT_ERR_INTERNAL, "path queue did not drain after %lld iterations", it);
                 }
                 PT_CHECK(r, cudaGraphLaunch(r->bounceGraph[it == 0 ? 0 : 1], s));
-                launches += 4 * (4 + extendKernels(false, inst, r->extendLane) + (slotOrdered(r) ? 1 : 0));
+                launches += 4 * (2 + extendKernels(false, inst, r->extendLane) + finalizeKernels(slotOrdered(r)));
                 r->profile.launches_extend += 4;
                 r->profile.launches_shadow += 4;
                 unsigned int live = 0;
@@ -1746,7 +1738,6 @@ int pt_render(pt_renderer* r, int waves)
                 }
                 {
                     StageTimer tm(r, kShade);
-                    launchShadeMiss(c, iter, sel, r->gridShadeMiss, nw, s);
                     launchShade(c, sel, iter, shadeGrid(r, nw), nw, s);
                 }
                 {
@@ -1755,12 +1746,9 @@ int pt_render(pt_renderer* r, int waves)
                 }
                 {
                     StageTimer tm(r, kFinalize);
-                    launchFinalize(c, sel, r->gridShadow, nw, s);
-                    if (slotOrdered(r)) {
-                        launchNextQueue(c, sel, r->gridShadow, s);
-                    }
+                    launchFinalize(c, sel, r->gridShadow, nw, slotOrdered(r), s);
                 }
-                launches += 4 + extendKernels(countVisits, inst, r->extendLane) + (slotOrdered(r) ? 1 : 0);
+                launches += 2 + extendKernels(countVisits, inst, r->extendLane) + finalizeKernels(slotOrdered(r));
                 r->profile.launches_extend += 1;
                 r->profile.launches_shadow += 1;
                 sel ^= 1;
@@ -2021,7 +2009,6 @@ int pt_set_tuning(pt_renderer* r, int path_capacity, int blocks_per_sm)
         r->gridShadowLane = r->smCount * std::min(blocks_per_sm, shadowLaneOccupancy());
         r->gridExtendLaneInst = r->smCount * std::min(blocks_per_sm, extendLaneInstOccupancy());
         r->gridShadowLaneInst = r->smCount * std::min(blocks_per_sm, shadowLaneInstOccupancy());
-        r->gridShadeMiss = r->smCount * std::min(blocks_per_sm, shadeMissOccupancy());
     } else {
         int be = 1, bs = 1, bsh = 1;
         stageOccupancy(be, bs, bsh);
@@ -2032,7 +2019,6 @@ int pt_set_tuning(pt_renderer* r, int path_capacity, int blocks_per_sm)
         r->gridShadowLane = r->smCount * shadowLaneOccupancy();
     r->gridExtendLaneInst = r->smCount * extendLaneInstOccupancy();
     r->gridShadowLaneInst = r->smCount * shadowLaneInstOccupancy();
-        r->gridShadeMiss = r->smCount * shadeMissOccupancy();
     }
     return PT_OK;
 }

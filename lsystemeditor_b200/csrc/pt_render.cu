@@ -952,9 +952,8 @@ __device__ __forceinline__ uint4 loadMarks(const uint8_t* flag, unsigned int k, 
     }
     return make_uint4(w[0], w[1], w[2], w[3]);
 }
-__global__ void __launch_bounds__(kListThreads) k_next_queue(const LaunchCtx* __restrict__ cp, int sel)
+__device__ __forceinline__ void listMarked(const LaunchCtx& c, int sel)
 {
-    const LaunchCtx& c = *cp;
     const unsigned int n = static_cast<unsigned int>(c.q.batch->slotCount);
     uint8_t* flag = c.q.nextFlag;
     uint32_t* out = c.q.extend[sel ^ 1];
@@ -1046,52 +1045,46 @@ __global__ void __launch_bounds__(kListThreads) k_next_queue(const LaunchCtx* __
     }
 }
 
-// Paths whose ray left the scene: previous bounce's NEE, then the
+// A path whose ray left the scene: previous bounce's NEE, then the
 // environment / background term (PathIntegratorRandCore.h:215-216, 338-346).
-#ifndef PT_SHADE_MISS_MIN_BLOCKS
-#define PT_SHADE_MISS_MIN_BLOCKS 4
-#endif
 template <int NW>
-__global__ void __launch_bounds__(256, PT_SHADE_MISS_MIN_BLOCKS) k_shade_miss(const LaunchCtx* __restrict__ cp, int iter, int sel)
+__device__ __forceinline__ void shadeMiss(const LaunchCtx& c, uint32_t i, unsigned int* nextCount, uint32_t* nextQueue)
 {
-    const LaunchCtx& c = *cp;
-    const unsigned int count = c.q.counts[4 + 2 * (iter & 1)];
-    unsigned int* nextCount = &c.q.counts[sel ^ 1];
-    uint32_t* nextQueue = c.q.extend[sel ^ 1];
-    for (unsigned int k = blockIdx.x * blockDim.x + threadIdx.x; k < count; k += gridDim.x * blockDim.x) {
-        const uint32_t i = c.q.missQueue[k];
-        const Waves<NW> wv = pathWaves<NW>(c, i);
-        const float4 d4 = c.paths.dir[i];
-        const float3 d = f3(d4.x, d4.y, d4.z);
-        const float4 r4 = c.paths.rad[i];
-        const int depth = __float_as_int(r4.w);
-        Col<NW> L;
-        const bool sunOn = c.sun.enabled != 0;
-        const bool black = skyIsBlack<NW>(c); // (adds exactly nothing)
-        if (depth == 0) {
-            L = black ? czero<NW>() : sunOn ? skyCol<NW>(c, d, wv) : envCol<NW>(c, d, wv);
-        } else {
-            L = loadCol<NW>(r4, c.paths.radS, c.paths.capacity, i);
-            if (c.paths.visEnv[i]) {
-                L = cadd(L, pendingEnv<NW>(c, i));
-            }
-            if (c.paths.visEmis[i]) {
-                L = cadd(L, pendingEmis<NW>(c, i));
-            }
-            if (!black) {
-                const Col<NW> T = loadCol<NW>(c.paths.thr[i], c.paths.thrS, c.paths.capacity, i);
-                const Col<NW> Le = sunOn ? skyCol<NW>(c, d, wv) : envCol<NW>(c, d, wv);
-                const float lp = sunOn ? skyPdf(c, d) : envPdf(c.env, d);
-                const float w = misBalance(fabsf(d4.w), lp);
-                L = cadd(L, cmul(T, cscl(Le, w)));
-            }
+    const Waves<NW> wv = pathWaves<NW>(c, i);
+    const float4 d4 = c.paths.dir[i];
+    const float3 d = f3(d4.x, d4.y, d4.z);
+    const float4 r4 = c.paths.rad[i];
+    const int depth = __float_as_int(r4.w);
+    Col<NW> L;
+    const bool sunOn = c.sun.enabled != 0;
+    const bool black = skyIsBlack<NW>(c); // (adds exactly nothing)
+    if (depth == 0) {
+        L = black ? czero<NW>() : sunOn ? skyCol<NW>(c, d, wv) : envCol<NW>(c, d, wv);
+    } else {
+        L = loadCol<NW>(r4, c.paths.radS, c.paths.capacity, i);
+        if (c.paths.visEnv[i]) {
+            L = cadd(L, pendingEnv<NW>(c, i));
         }
-        writeSample<NW>(c, i, L, wv);
-        recyclePath<NW>(c, i, nextCount, nextQueue);
+        if (c.paths.visEmis[i]) {
+            L = cadd(L, pendingEmis<NW>(c, i));
+        }
+        if (!black) {
+            const Col<NW> T = loadCol<NW>(c.paths.thr[i], c.paths.thrS, c.paths.capacity, i);
+            const Col<NW> Le = sunOn ? skyCol<NW>(c, d, wv) : envCol<NW>(c, d, wv);
+            const float lp = sunOn ? skyPdf(c, d) : envPdf(c.env, d);
+            const float w = misBalance(fabsf(d4.w), lp);
+            L = cadd(L, cmul(T, cscl(Le, w)));
+        }
     }
+    writeSample<NW>(c, i, L, wv);
+    recyclePath<NW>(c, i, nextCount, nextQueue);
 }
 
-// Shading of the paths that hit a triangle. One thread per queued path.
+// Shading of the paths that hit a triangle, then of those that left the scene.
+// One thread per queued path.  (The misses in this launch and not in one of
+// their own: they start in the blocks that the hits leave idle, and a bounce of
+// few paths has one launch less: 4 waves of 1024^2 pixels 7.1 -> 6.97 ms with the
+// merged listing pass below.)
 //
 // Bound by instruction fetch: a path runs through about 30 KB of straight-line
 // code (the kernel has 170 - 230 KB), and with warps spread over it a third of
@@ -1480,6 +1473,10 @@ __global__ void __launch_bounds__(kShadeThreads, PT_SHADE_MIN_BLOCKS)
                 c.paths.visEmis[i] = 0;
             }
         }
+    }    const unsigned int misses = c.q.counts[4 + 2 * (iter & 1)];
+    for (unsigned int k = (gridDim.x - 1u - blockIdx.x) * blockDim.x + threadIdx.x; k < misses;
+         k += gridDim.x * blockDim.x) {
+        shadeMiss<NW>(c, c.q.missQueue[k], nextCount, nextQueue);
     }
 }
 
@@ -1523,9 +1520,11 @@ __global__ void __launch_bounds__(256, 4) k_shadow(const LaunchCtx* __restrict__
     }
 }
 
-// Paths that terminated while their NEE shadow rays were in flight.
-template <int NW>
-__global__ void __launch_bounds__(256) k_finalize(const LaunchCtx* __restrict__ cp, int sel)
+// Paths that terminated while their NEE shadow rays were in flight; in
+// slot-ordered mode also the next bounce's extend queue (List; with path
+// generations nothing here marks a slot).
+template <int NW, bool List>
+__global__ void __launch_bounds__(kListThreads) k_finalize(const LaunchCtx* __restrict__ cp, int sel)
 {
     const LaunchCtx& c = *cp;
     const unsigned int count = c.q.counts[3];
@@ -1543,8 +1542,13 @@ __global__ void __launch_bounds__(256) k_finalize(const LaunchCtx* __restrict__ 
         }
         writeSample<NW>(c, i, L, wv);
         recyclePath<NW>(c, i, nextCount, nextQueue);
+    }    if constexpr (List) {
+        listMarked(c, sel);
     }
 }
+#if !PT_PATH_GENERATIONS
+__global__ void __launch_bounds__(kListThreads) k_next_queue(const LaunchCtx* __restrict__ cp, int sel) { listMarked(*cp, sel); }
+#endif
 
 // Per pixel: fold the batch's samples in sample order (PathTracer.cu:232-272).
 __global__ void __launch_bounds__(256) k_accumulate(const LaunchCtx* __restrict__ cp, int activeCount, int batch)
@@ -1828,10 +1832,6 @@ int extendKernels(bool count, bool inst, bool lane)
 {
     return (!count && lane) ? 2 : 1;
 }
-void launchNextQueue(const LaunchCtx* c, int sel, int grid, cudaStream_t s)
-{
-    k_next_queue<<<grid, kListThreads, 0, s>>>(c, sel);
-}
 int extendLaneOccupancy()
 {
     return blocksPerSm(k_extend_lane<false, false>, kTraceThreads, traceSmemBytes<false>());
@@ -1847,22 +1847,6 @@ int shadowLaneOccupancy()
 int shadowLaneInstOccupancy()
 {
     return blocksPerSm(k_shadow_lane<true, false>, kTraceThreads, traceSmemBytes<true>());
-}
-int shadeMissOccupancy()
-{
-    int blocks = 1;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k_shade_miss<8>, 256, 0);
-    return blocks > 0 ? blocks : 1;
-}
-void launchShadeMiss(const LaunchCtx* c, int iter, int sel, int grid, int nw, cudaStream_t s)
-{
-    if (nw == 8) {
-        k_shade_miss<8><<<grid, 256, 0, s>>>(c, iter, sel);
-    } else if (nw == 4) {
-        k_shade_miss<4><<<grid, 256, 0, s>>>(c, iter, sel);
-    } else {
-        k_shade_miss<0><<<grid, 256, 0, s>>>(c, iter, sel);
-    }
 }
 void launchShade(const LaunchCtx* c, int sel, int iter, int grid, int nw, cudaStream_t s)
 {
@@ -1926,16 +1910,34 @@ void stageOccupancy(int& extendBlocks, int& shadeBlocks, int& shadowBlocks)
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&shadeBlocks, k_shade<0>, kShadeThreads, 0);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&shadowBlocks, k_shadow<false, false>, 256, smem);
 }
-void launchFinalize(const LaunchCtx* c, int sel, int grid, int nw, cudaStream_t s)
+namespace {
+template <int NW> void finalize(const LaunchCtx* c, int sel, int grid, bool list, cudaStream_t s)
+{
+#if PT_PATH_GENERATIONS
+    if (list) {
+        k_finalize<NW, true><<<grid, kListThreads, 0, s>>>(c, sel);
+        return;
+    }
+#endif
+    k_finalize<NW, false><<<grid, kListThreads, 0, s>>>(c, sel);
+#if !PT_PATH_GENERATIONS
+    if (list) {
+        k_next_queue<<<grid, kListThreads, 0, s>>>(c, sel);
+    }
+#endif
+}
+} // namespace
+void launchFinalize(const LaunchCtx* c, int sel, int grid, int nw, bool list, cudaStream_t s)
 {
     if (nw == 8) {
-        k_finalize<8><<<grid, 256, 0, s>>>(c, sel);
+        finalize<8>(c, sel, grid, list, s);
     } else if (nw == 4) {
-        k_finalize<4><<<grid, 256, 0, s>>>(c, sel);
+        finalize<4>(c, sel, grid, list, s);
     } else {
-        k_finalize<0><<<grid, 256, 0, s>>>(c, sel);
+        finalize<0>(c, sel, grid, list, s);
     }
 }
+int finalizeKernels(bool list) { return list && !PT_PATH_GENERATIONS ? 2 : 1; }
 void launchAccumulate(const LaunchCtx* c, int activeCount, int batch, cudaStream_t s)
 {
     k_accumulate<<<gridFor(activeCount), 256, 0, s>>>(c, activeCount, batch);

@@ -160,7 +160,7 @@ struct LaunchCtx {
 // passed by pointer: a large by-value kernel parameter whose members are
 // taken by reference would be copied to local memory by every thread.
 // `grid` is a persistent-style grid; kernels loop over device-side counts.
-// `nw` (generate, shade-miss, shade, finalize): wavelengths per path, 0 = RGB.
+// `nw` (generate, shade, finalize): wavelengths per path, 0 = RGB.
 void launchGenerate(const LaunchCtx* d, int count, int extendSel, int nw, cudaStream_t s,
     unsigned long long jobOffset = 0);
 // inst: compile-time instanced-scene traversal (any scene of the context instanced).
@@ -170,22 +170,21 @@ void launchExtend(const LaunchCtx* d, int sel, bool identity, int iter, int grid
     bool multi, cudaStream_t s);
 // Kernels one launchExtend call launches (closest hit, and the routing pass after it).
 int extendKernels(bool count, bool inst, bool lane);
-// Resident blocks per SM of the per-lane closest-hit kernel and of the miss shader.
+// Resident blocks per SM of the per-lane kernels.
 int extendLaneOccupancy();
-int shadeMissOccupancy();
 int shadowLaneOccupancy();
 int extendLaneInstOccupancy();
 int shadowLaneInstOccupancy();
-// Resident blocks per SM of the hit shader for nw wavelengths (0 = RGB).
+// Resident blocks per SM of the shade kernel for nw wavelengths (0 = RGB).
 int shadeOccupancy(int nw);
-// Slot-ordered mode: the next bounce's extend queue from the marked slots.
-void launchNextQueue(const LaunchCtx* d, int sel, int grid, cudaStream_t s);
-void launchShadeMiss(const LaunchCtx* d, int iter, int sel, int grid, int nw, cudaStream_t s);
 void launchShade(const LaunchCtx* d, int sel, int iter, int grid, int nw, cudaStream_t s);
 // Shadow stage.  lane: per-lane ray replacement (k_shadow_lane; flat scenes,
 // no visit counting), else one warp per 32 queued rays (k_shadow).
 void launchShadow(const LaunchCtx* d, int iter, int grid, bool count, bool inst, bool lane, bool multi, cudaStream_t s);
-void launchFinalize(const LaunchCtx* d, int sel, int grid, int nw, cudaStream_t s);
+// list: slot-ordered mode, the next bounce's extend queue from the marked slots.
+void launchFinalize(const LaunchCtx* d, int sel, int grid, int nw, bool list, cudaStream_t s);
+// Kernels one launchFinalize call launches.
+int finalizeKernels(bool list);
 void launchAccumulate(const LaunchCtx* d, int activeCount, int batch, cudaStream_t s);
 // Stable compaction of the active list (pixels neither converged nor at the
 // sample cap), so that the list stays sorted by pixel and thereby by scene.
