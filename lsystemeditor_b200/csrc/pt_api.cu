@@ -10,6 +10,7 @@
 #include "pt_output.cuh"
 #include "pt_scene.cuh"
 #include "pt_spectral.cuh"
+#include "pt_hostcopy.cuh"
 
 namespace pt {
 // pt_l2probe.cu
@@ -20,6 +21,7 @@ int measureL2ReadBandwidth(size_t bytes, int reps, int smCount, cudaStream_t s, 
 #include <array>
 #include <cmath>
 #include <map>
+#include <memory>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
@@ -205,6 +207,10 @@ struct pt_renderer {
     int previewLevels = 0;
     int previewDone = -1;                 // finest preview level rendered since the last reset
     DevBuf<float4> previewBuf;            // all levels, coarsest first
+    DevBuf<char> queryBuf;                // inputs and results of pt_trace_rays
+    std::unique_ptr<HostCopier> copier;   // staged copies from and to pageable memory
+    cudaStream_t copyStream = nullptr;    // uploads beside the work on `stream`
+    cudaEvent_t copyEvent = nullptr;      // orders the two
     // region render (PathTracer.h:134-140)
     bool regionEnabled = false;
     int regionMinX = 0, regionMinY = 0, regionMaxX = 0, regionMaxY = 0;
@@ -950,7 +956,9 @@ int buildEmissive(pt_renderer* r, SceneSlot& sl, uint32_t n)
 // With the triangles of a scene in sl.positions (9 floats each) and their
 // normals, uvs and material ids in the staging buffers: shading records, the
 // emissive list and CDF, and the BVH, all on the device.
-int finishScene(pt_renderer* r, SceneSlot& sl, uint32_t n)
+// uploading: the normals and uvs are on their way on copyStream; the shading
+// records, which nothing else of the build reads, then come last.
+int finishScene(pt_renderer* r, SceneSlot& sl, uint32_t n, bool uploading = false)
 {
     cudaStream_t s = r->stream;
     sl.triCount = n;
@@ -966,8 +974,10 @@ int finishScene(pt_renderer* r, SceneSlot& sl, uint32_t n)
     if (!sl.shade.ensure(n)) {
         return fail(r, PT_ERR_OUT_OF_MEMORY, "shading records allocation failed for %u triangles", n);
     }
-    launchBuildShade(r->stage.p, r->stage.p + 9ull * n, r->stageIds.p, n, sl.shade.p, s);
-    PT_CHECK(r, cudaGetLastError());
+    if (!uploading) {
+        launchBuildShade(r->stage.p, r->stage.p + 9ull * n, r->stageIds.p, n, sl.shade.p, s);
+        PT_CHECK(r, cudaGetLastError());
+    }
     {
         const int st = buildEmissive(r, sl, n);
         if (st != PT_OK) {
@@ -978,6 +988,13 @@ int finishScene(pt_renderer* r, SceneSlot& sl, uint32_t n)
     const int st = buildBvh(sl.positions.p, n, sl.bvh, s, r->bvhOptions, err, sizeof(err));
     if (st != PT_OK) {
         return fail(r, st, "BVH build: %s", err);
+    }
+    if (uploading) {
+        PT_CHECK(r, r->copier->finish());
+        PT_CHECK(r, cudaEventRecord(r->copyEvent, r->copyStream));
+        PT_CHECK(r, cudaStreamWaitEvent(s, r->copyEvent, 0));
+        launchBuildShade(r->stage.p, r->stage.p + 9ull * n, r->stageIds.p, n, sl.shade.p, s);
+        PT_CHECK(r, cudaGetLastError());
     }
     return PT_OK;
 }
@@ -1011,14 +1028,23 @@ int setSceneMesh(pt_renderer* r, SceneSlot& sl, const pt_mesh* mesh)
         if (!sl.positions.ensure(9ull * n) || !r->stage.ensure(15ull * n) || !r->stageIds.ensure(n)) {
             return fail(r, PT_ERR_OUT_OF_MEMORY, "mesh upload failed for %u triangles", n);
         }
-        PT_CHECK(r, cudaMemcpyAsync(sl.positions.p, mesh->positions, 9ull * n * sizeof(float), cudaMemcpyHostToDevice, s));
-        PT_CHECK(r, cudaMemcpyAsync(r->stage.p, mesh->normals, 9ull * n * sizeof(float), cudaMemcpyHostToDevice, s));
-        PT_CHECK(r, cudaMemcpyAsync(r->stage.p + 9ull * n, mesh->uvs, 6ull * n * sizeof(float), cudaMemcpyHostToDevice, s));
-        PT_CHECK(r, cudaMemcpyAsync(r->stageIds.p, mesh->material_ids, n * sizeof(uint32_t), cudaMemcpyHostToDevice, s));
+        // the build starts with the positions and ids; the normals and uvs are
+        // uploaded beside it
+        const HostCopier::Piece first[2] = {{sl.positions.p, const_cast<float*>(mesh->positions), 9ull * n * sizeof(float)},
+            {r->stageIds.p, const_cast<uint32_t*>(mesh->material_ids), n * sizeof(uint32_t)}};
+        const HostCopier::Piece second[2] = {{r->stage.p, const_cast<float*>(mesh->normals), 9ull * n * sizeof(float)},
+            {r->stage.p + 9ull * n, const_cast<float*>(mesh->uvs), 6ull * n * sizeof(float)}};
+        PT_CHECK(r, cudaEventRecord(r->copyEvent, s));
+        PT_CHECK(r, cudaStreamWaitEvent(r->copyStream, r->copyEvent, 0));
+        PT_CHECK(r, r->copier->beginUpload(first, 2, s));
+        PT_CHECK(r, r->copier->finish());
+        PT_CHECK(r, r->copier->beginUpload(second, 2, r->copyStream));
     }
     {
-        const int st = finishScene(r, sl, n);
+        const int st = finishScene(r, sl, n, n > 0);
         if (st != PT_OK) {
+            r->copier->finish(); // (the caller's arrays are not read after the call)
+            cudaStreamSynchronize(r->copyStream);
             return st;
         }
     }
@@ -1328,11 +1354,14 @@ int pt_create(pt_renderer** out, int device)
     }
     if (cudaSetDevice(r->device) != cudaSuccess ||
         cudaStreamCreateWithFlags(&r->ownStream, cudaStreamNonBlocking) != cudaSuccess ||
+        cudaStreamCreateWithFlags(&r->copyStream, cudaStreamNonBlocking) != cudaSuccess ||
+        cudaEventCreateWithFlags(&r->copyEvent, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreate(&r->ev0) != cudaSuccess || cudaEventCreate(&r->ev1) != cudaSuccess) {
         delete r;
         return PT_ERR_CUDA;
     }
     r->stream = r->ownStream;
+    r->copier.reset(new HostCopier(r->device));
     cudaDeviceGetAttribute(&r->smCount, cudaDevAttrMultiProcessorCount, r->device);
     pt_default_params(&r->params);
     r->scenes[0].camera = defaultCamera();
@@ -1357,6 +1386,14 @@ int pt_destroy(pt_renderer* r)
     cudaSetDevice(r->device);
     if (r->stream) {
         cudaStreamSynchronize(r->stream);
+    }
+    r->copier.reset();
+    if (r->copyStream) {
+        cudaStreamSynchronize(r->copyStream);
+        cudaStreamDestroy(r->copyStream);
+    }
+    if (r->copyEvent) {
+        cudaEventDestroy(r->copyEvent);
     }
     for (SceneSlot& sl : r->scenes) {
         sl.release();
@@ -1404,6 +1441,7 @@ int pt_destroy(pt_renderer* r)
     r->adjImage.release();
     r->record.release();
     r->previewBuf.release();
+    r->queryBuf.release();
     r->adjGrad.release();
     r->compactTemp.release();
     r->sceneActiveStart.release();
@@ -1913,13 +1951,16 @@ int pt_trace_rays(pt_renderer* r, int n, const float* origins, const float* dirs
     }
     PT_CHECK(r, cudaSetDevice(r->device));
     const size_t N = static_cast<size_t>(n);
-    // one staging allocation: inputs 8 floats, outputs 1 byte + 7 words per ray
+    // one buffer, kept for the next query: inputs 8 floats, outputs 1 byte + 7 words per ray
     const size_t bytes = N * (8 * sizeof(float) + 7 * sizeof(float) + 16);
-    void* buf = nullptr;
-    PT_CHECK(r, cudaMallocAsync(&buf, bytes + 16, r->stream));
+    if (!r->queryBuf.ensure(bytes + 32)) {
+        cudaGetLastError();
+        return fail(r, PT_ERR_OUT_OF_MEMORY, "pt_trace_rays: %d rays do not fit", n);
+    }
+    char* buf = r->queryBuf.p;
     // traversal stack overflows of this query (pt_stats.stack_overflows)
-    unsigned int* dOverflow = reinterpret_cast<unsigned int*>(static_cast<char*>(buf) + ((bytes + 15) & ~size_t(15)));
-    float* dO = static_cast<float*>(buf);
+    unsigned int* dOverflow = reinterpret_cast<unsigned int*>(buf + ((bytes + 15) & ~size_t(15)));
+    float* dO = reinterpret_cast<float*>(buf);
     float* dD = dO + 3 * N;
     float* dTmin = dD + 3 * N;
     float* dTmax = dTmin + N;
@@ -1932,21 +1973,32 @@ int pt_trace_rays(pt_renderer* r, int n, const float* origins, const float* dirs
     int rc = PT_OK;
     unsigned int overflow = 0;
     cudaError_t e = cudaMemsetAsync(dOverflow, 0, sizeof(unsigned int), s);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(dO, origins, 3 * N * sizeof(float), cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(dD, dirs, 3 * N * sizeof(float), cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(dTmin, tmin, N * sizeof(float), cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(dTmax, tmax, N * sizeof(float), cudaMemcpyHostToDevice, s);
+    const HostCopier::Piece in[4] = {{dO, const_cast<float*>(origins), 3 * N * sizeof(float)},
+        {dD, const_cast<float*>(dirs), 3 * N * sizeof(float)}, {dTmin, const_cast<float*>(tmin), N * sizeof(float)},
+        {dTmax, const_cast<float*>(tmax), N * sizeof(float)}};
+    if (e == cudaSuccess) e = r->copier->beginUpload(in, 4, s);
+    const cudaError_t copied = r->copier->finish();
+    if (e == cudaSuccess) e = copied;
     if (e == cudaSuccess) {
         launchTraceRays(deviceScene(&r->scenes[0]), n, dO, dD, dTmin, dTmax, dHit, dT, dTri, dN, dUv, s, dOverflow);
         e = cudaGetLastError();
     }
+    HostCopier::Piece out[5];
+    size_t pieces = 0;
+    auto give = [&](void* device, void* host, size_t size) {
+        if (host != nullptr) {
+            out[pieces++] = HostCopier::Piece{device, host, size};
+        }
+    };
+    give(dHit, hit, N);
+    give(dT, t, N * sizeof(float));
+    give(dTri, tri, N * sizeof(uint32_t));
+    give(dN, normal, 3 * N * sizeof(float));
+    give(dUv, uv, 2 * N * sizeof(float));
     if (e == cudaSuccess) e = cudaMemcpyAsync(&overflow, dOverflow, sizeof(overflow), cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(hit, dHit, N, cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess && t) e = cudaMemcpyAsync(t, dT, N * sizeof(float), cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess && tri) e = cudaMemcpyAsync(tri, dTri, N * sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess && normal) e = cudaMemcpyAsync(normal, dN, 3 * N * sizeof(float), cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess && uv) e = cudaMemcpyAsync(uv, dUv, 2 * N * sizeof(float), cudaMemcpyDeviceToHost, s);
-    cudaFreeAsync(buf, s);
+    if (e == cudaSuccess) e = r->copier->beginDownload(out, pieces, s);
+    const cudaError_t landed = r->copier->finish();
+    if (e == cudaSuccess) e = landed;
     const cudaError_t e2 = cudaStreamSynchronize(s);
     if (e == cudaSuccess) {
         e = e2;

@@ -99,3 +99,28 @@ def test_more_slots_than_one_step_per_warp(tracer):
     tracer.set_extend_mode(0)
     for a, b in zip(*out):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("n", [1, 130_000, 131_073, 300_001])
+def test_ray_queries_through_staged_copies(tracer, n):
+    """Queries on both sides of the size from which host arrays are staged through pinned slices (4 MB in: 131072
+    rays), with partial last slices, give what one query of the same rays in small parts gives."""
+    mesh = zoo_scene(n_per_mat=30, seed=5)
+    tracer.configure(8, 8, mesh)
+    o, d = rays_through_bounds(mesh, n, seed=7)
+    for _ in range(3):  # (transfers of this size are staged from the fifth on: two per query)
+        whole = tracer.trace_rays(o, d)
+    parts = [tracer.trace_rays(o[a:a + 60_000], d[a:a + 60_000]) for a in range(0, n, 60_000)]
+    for k, v in whole.items():
+        assert np.array_equal(v, np.concatenate([p[k] for p in parts])), k
+
+
+@pytest.mark.parametrize("n", [40_000, 559_241, 900_001])
+def test_staged_mesh_upload(tracer, n):
+    """A mesh comes back bit for bit below and above the size (32 MB of normals and uvs) from which its arrays are
+    staged through pinned slices at once."""
+    mesh = random_soup(n, seed=2, extent=30.0, size=0.2, materials=3)
+    tracer.configure(8, 8, mesh)
+    back = tracer.export_mesh()
+    for name in ("positions", "normals", "uvs", "material_ids"):
+        assert np.array_equal(getattr(back, name), getattr(mesh, name)), name
