@@ -239,9 +239,9 @@ struct pt_renderer {
     DevBuf<uint32_t> qExt0, qExt1, qFinish, qShadowPath, qMiss, qHit;
     DevBuf<float4> qShadowO, qShadowD;
     DevBuf<unsigned int> qCounts;
-    DevBuf<unsigned long long> qRays;     // [0] extend, [1] shadow
-    DevBuf<unsigned long long> qVisits;   // [0..1] extend nodes/tris, [2..3] shadow nodes/tris
-    DevBuf<unsigned int> qOverflow;
+    // counters of a render: rays (extend, shadow), visits (extend nodes and tris,
+    // shadow nodes and tris), traversal stack overflows (32 bits)
+    DevBuf<unsigned long long> qStats;
     int gridExtend = 0, gridShade = 0, gridShadow = 0;
     int gridExtendLane = 0;          // grid of the per-lane closest-hit kernel
     int gridShadowLane = 0;          // grid of the per-lane shadow kernel
@@ -378,8 +378,8 @@ int ensurePaths(pt_renderer* r, int capacity)
         r->pNeeEnv.ensure(Q) && r->pNeeEmis.ensure(Q) && r->pVisEnv.ensure(Q) && r->pVisEmis.ensure(Q) && r->pScene.ensure(Q) &&
         r->qExt0.ensure(Q) && r->qExt1.ensure(Q) && r->qFinish.ensure(Q) && r->qShadowPath.ensure(2 * Q) &&
         r->qMiss.ensure(Q) && r->qHit.ensure(Q) &&
-        r->qShadowO.ensure(2 * Q) && r->qShadowD.ensure(2 * Q) && r->qCounts.ensure(16) && r->qRays.ensure(2) &&
-        r->qVisits.ensure(4) && r->qOverflow.ensure(1) && r->dbatch.ensure(1) && r->pNextFlag.ensure(Q);
+        r->qShadowO.ensure(2 * Q) && r->qShadowD.ensure(2 * Q) && r->qCounts.ensure(16) && r->qStats.ensure(7) &&
+        r->dbatch.ensure(1) && r->pNextFlag.ensure(Q);
     if (!ok) {
         return fail(r, PT_ERR_OUT_OF_MEMORY, "path state allocation failed for %d paths", capacity);
     }
@@ -452,10 +452,10 @@ LaunchCtx makeCtx(pt_renderer* r)
     c.q.shadowOrig = r->qShadowO.p;
     c.q.shadowDir = r->qShadowD.p;
     c.q.counts = r->qCounts.p;
-    c.q.rays = r->qRays.p;
+    c.q.rays = r->qStats.p;
     c.q.batch = r->dbatch.p;
-    c.q.visits = r->qVisits.p;
-    c.q.overflow = r->qOverflow.p;
+    c.q.visits = r->qStats.p + 2;
+    c.q.overflow = reinterpret_cast<unsigned int*>(r->qStats.p + 6);
     c.acc.acc = r->acc.p;
     c.acc.counts = r->counts.p;
     c.acc.lumMean = r->lumMean.p;
@@ -1471,9 +1471,7 @@ int pt_destroy(pt_renderer* r)
     r->qShadowO.release();
     r->qShadowD.release();
     r->qCounts.release();
-    r->qRays.release();
-    r->qVisits.release();
-    r->qOverflow.release();
+    r->qStats.release();
     r->dctx.release();
     r->dbatch.release();
     releaseBounceGraphs(r);
@@ -1699,9 +1697,7 @@ int pt_render(pt_renderer* r, int waves)
     const bool countVisits = (r->profileFlags & PT_PROFILE_COUNT_VISITS) != 0;
     r->profile = pt_profile{};
     r->eventMarks.clear();
-    PT_CHECK(r, cudaMemsetAsync(r->qRays.p, 0, 2 * sizeof(unsigned long long), s));
-    PT_CHECK(r, cudaMemsetAsync(r->qVisits.p, 0, 4 * sizeof(unsigned long long), s));
-    PT_CHECK(r, cudaMemsetAsync(r->qOverflow.p, 0, sizeof(unsigned int), s));
+    PT_CHECK(r, cudaMemsetAsync(r->qStats.p, 0, 7 * sizeof(unsigned long long), s));
     PT_CHECK(r, cudaEventRecord(r->ev0, s));
     int remaining = waves;
     int64_t launches = 0;
@@ -1804,12 +1800,16 @@ int pt_render(pt_renderer* r, int waves)
             }
         }
         PT_CHECK(r, cudaGetLastError());
+        PT_CHECK(r, cudaMemsetAsync(r->activeCount.p + 1, 0, sizeof(int), s));
         {
             StageTimer tm(r, kAccumulate);
             launchAccumulate(c, active, B, s);
         }
-        PT_CHECK(r, cudaMemsetAsync(r->activeCount.p + 1, 0, sizeof(int), s));
-        {
+        ++launches;
+        int next = 0; // pixels that go on
+        PT_CHECK(r, cudaMemcpyAsync(&next, r->activeCount.p + 1, sizeof(int), cudaMemcpyDeviceToHost, s));
+        PT_CHECK(r, cudaStreamSynchronize(s));
+        if (next > 0 && next < active) {
             StageTimer tm(r, kCompact);
             const size_t tb = compactTempBytes(active);
             if (!r->compactTemp.ensure(tb)) {
@@ -1818,14 +1818,11 @@ int pt_render(pt_renderer* r, int waves)
             int* lists[2] = {r->active0.p, r->active1.p};
             PT_CHECK(r, launchCompactStable(lists[r->activeSel], lists[r->activeSel ^ 1], r->activeCount.p + 1, active,
                 r->converged.p, r->counts.p, r->params.max_samples_per_pixel, r->compactTemp.p, tb, s));
+            r->activeSel ^= 1;
+            ++launches;
         }
-        launches += 2;
-        int next = 0;
-        PT_CHECK(r, cudaMemcpyAsync(&next, r->activeCount.p + 1, sizeof(int), cudaMemcpyDeviceToHost, s));
-        PT_CHECK(r, cudaStreamSynchronize(s));
         PT_CHECK(r, cudaGetLastError());
         r->lastStopRate = static_cast<double>(active - next) / active / std::max(1.0, B / 4.0);
-        r->activeSel ^= 1;
         r->hostActive = next;
         r->wavesDone += B;
         r->samplesDone += jobs;
@@ -1839,15 +1836,13 @@ int pt_render(pt_renderer* r, int waves)
         r->wavesDone >= r->recordSpp && r->params.min_samples == r->recordSpp &&
         r->params.max_samples_per_pixel == r->recordSpp;
     PT_CHECK(r, cudaEventRecord(r->ev1, s));
-    PT_CHECK(r, cudaEventSynchronize(r->ev1));
+    unsigned long long stats[7] = {};
+    PT_CHECK(r, cudaMemcpyAsync(stats, r->qStats.p, sizeof(stats), cudaMemcpyDeviceToHost, s));
+    PT_CHECK(r, cudaStreamSynchronize(s));
     float ms = 0.0f;
     cudaEventElapsedTime(&ms, r->ev0, r->ev1);
-    unsigned long long rays[2] = {0, 0};
-    unsigned long long visits[4] = {0, 0, 0, 0};
-    unsigned int overflow = 0;
-    PT_CHECK(r, cudaMemcpy(rays, r->qRays.p, sizeof(rays), cudaMemcpyDeviceToHost));
-    PT_CHECK(r, cudaMemcpy(visits, r->qVisits.p, sizeof(visits), cudaMemcpyDeviceToHost));
-    PT_CHECK(r, cudaMemcpy(&overflow, r->qOverflow.p, sizeof(overflow), cudaMemcpyDeviceToHost));
+    const unsigned long long *rays = stats, *visits = stats + 2;
+    const unsigned int overflow = static_cast<unsigned int>(stats[6]);
     collectStageTimes(r);
     r->profile.rays_extend = static_cast<int64_t>(rays[0]);
     r->profile.rays_shadow = static_cast<int64_t>(rays[1]);

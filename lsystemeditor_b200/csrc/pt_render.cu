@@ -1551,7 +1551,11 @@ __global__ void __launch_bounds__(kListThreads) k_next_queue(const LaunchCtx* __
 #endif
 
 // Per pixel: fold the batch's samples in sample order (PathTracer.cu:232-272).
-__global__ void __launch_bounds__(256) k_accumulate(const LaunchCtx* __restrict__ cp, int activeCount, int batch)
+// activeCount[1] counts the pixels that go on (KeepActive), so that the list is
+// compacted only when some pixels stopped and some did not: three launches less
+// for a wave in which none stops and for a render's last batch.
+constexpr int kAccumulateThreads = 256;
+__global__ void __launch_bounds__(kAccumulateThreads) k_accumulate(const LaunchCtx* __restrict__ cp, int activeCount, int batch)
 {
     const LaunchCtx& c = *cp;
     const int* active = c.acc.active[c.activeSel];
@@ -1562,6 +1566,7 @@ __global__ void __launch_bounds__(256) k_accumulate(const LaunchCtx* __restrict_
     // criterion 2: a pixel all of whose samples are black stops after max(min spp, 64) samples
     const bool blackStops = c.params.adaptive_criterion == 2;
     const uint32_t blackSpp = static_cast<uint32_t>(minSpp > 64 ? minSpp : 64);
+    unsigned int kept = 0;
     for (int li = blockIdx.x * blockDim.x + threadIdx.x; li < activeCount; li += gridDim.x * blockDim.x) {
         const int p = active[li];
         uint8_t conv = c.acc.converged[p];
@@ -1614,6 +1619,21 @@ __global__ void __launch_bounds__(256) k_accumulate(const LaunchCtx* __restrict_
         c.acc.m2[p] = m2;
         c.acc.acc[p] = a;
         c.acc.converged[p] = conv;
+        kept += conv == 0 && !(maxSpp > 0 && n >= static_cast<uint32_t>(maxSpp)) ? 1u : 0u;
+    }
+    __shared__ unsigned int sKept[kAccumulateThreads / 32];
+    kept = __reduce_add_sync(0xffffffffu, kept);
+    if ((threadIdx.x & 31) == 0) {
+        sKept[threadIdx.x >> 5] = kept;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < kAccumulateThreads / 32; ++w) {
+            kept += sKept[w];
+        }
+        if (kept != 0u) {
+            atomicAdd(&c.acc.activeCount[1], static_cast<int>(kept));
+        }
     }
 }
 
@@ -1940,7 +1960,7 @@ void launchFinalize(const LaunchCtx* c, int sel, int grid, int nw, bool list, cu
 int finalizeKernels(bool list) { return list && !PT_PATH_GENERATIONS ? 2 : 1; }
 void launchAccumulate(const LaunchCtx* c, int activeCount, int batch, cudaStream_t s)
 {
-    k_accumulate<<<gridFor(activeCount), 256, 0, s>>>(c, activeCount, batch);
+    k_accumulate<<<gridFor(activeCount, kAccumulateThreads), kAccumulateThreads, 0, s>>>(c, activeCount, batch);
 }
 size_t compactTempBytes(int n)
 {
