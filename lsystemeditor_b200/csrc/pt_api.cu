@@ -1309,7 +1309,7 @@ bool ensureBounceGraphs(pt_renderer* r, const LaunchCtx* c, bool inst, int nw)
         int sel = 0;
         for (int it = 0; it < 4; ++it) {
             launchExtend(c, sel, g == 0 && it == 0, it, extendGrid(r, false, inst), false, inst, r->extendLane, r->scenes.size() > 1, s);
-            launchShade(c, sel, it, shadeGrid(r, nw), nw, s);
+            launchShade(c, sel, it, g == 0 && it == 0, shadeGrid(r, nw), nw, s);
             launchShadow(c, it, shadowGrid(r, false, inst), false, inst, r->extendLane, r->scenes.size() > 1, s);
             launchFinalize(c, sel, r->gridShadow, nw, slotOrdered(r), s);
             sel ^= 1;
@@ -1718,10 +1718,6 @@ int pt_render(pt_renderer* r, int waves)
         r->hbatch.activeCount = active;
         r->hbatch.waveBase = static_cast<uint32_t>(r->wavesDone);
         r->hbatch.slotCount = slots;
-        if (slotOrdered(r)) {
-            // (marks are cleared by k_next_queue; this also clears those of a render that failed)
-            PT_CHECK(r, cudaMemsetAsync(r->pNextFlag.p, 0, static_cast<size_t>(slots), s));
-        }
         PT_CHECK(r, cudaMemcpyAsync(r->dbatch.p, &r->hbatch, sizeof(BatchInfo), cudaMemcpyHostToDevice, s));
         const LaunchCtx* c = uploadCtx(r);
         if (c == nullptr) {
@@ -1772,7 +1768,7 @@ int pt_render(pt_renderer* r, int waves)
                 }
                 {
                     StageTimer tm(r, kShade);
-                    launchShade(c, sel, iter, shadeGrid(r, nw), nw, s);
+                    launchShade(c, sel, iter, it == 0, shadeGrid(r, nw), nw, s);
                 }
                 {
                     StageTimer tm(r, kShadow);
@@ -1800,7 +1796,6 @@ int pt_render(pt_renderer* r, int waves)
             }
         }
         PT_CHECK(r, cudaGetLastError());
-        PT_CHECK(r, cudaMemsetAsync(r->activeCount.p + 1, 0, sizeof(int), s));
         {
             StageTimer tm(r, kAccumulate);
             launchAccumulate(c, active, B, s);

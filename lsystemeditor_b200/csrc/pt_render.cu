@@ -572,15 +572,19 @@ template <int NW> __device__ __forceinline__ void initPath(const LaunchCtx& c, u
     rngStore(c.paths, i, st);
     c.paths.orig[i] = make_float4(ro.x, ro.y, ro.z, 0.0f);
     c.paths.dir[i] = make_float4(rd.x, rd.y, rd.z, 0.0f);
+    // The throughput, radiance, depth and next-event flags of a path at depth 0
+    // are 1, 0, 0 and clear: with path generations a whole launch is at depth 0
+    // and they are not stored (generation is bound by its writes: 16.7M paths
+    // 329 -> 281 us).
+#if !PT_PATH_GENERATIONS
     c.paths.thr[i] = make_float4(1.0f, 1.0f, 1.0f, 1.0f);
     c.paths.rad[i] = make_float4(0.0f, 0.0f, 0.0f, __int_as_float(0));
-    if constexpr (NW > 0) {
-        // (the spectral throughput and radiance of a path at depth 0 are 1 and
-        // 0: they are not stored, the shade kernels know them)
-        c.paths.hero[i] = spectral::heroU(seed);
-    }
     c.paths.visEnv[i] = 0;
     c.paths.visEmis[i] = 0;
+#endif
+    if constexpr (NW > 0) {
+        c.paths.hero[i] = spectral::heroU(seed);
+    }
 }
 
 // Path i joins the next bounce's extend queue: marked for k_next_queue in
@@ -639,9 +643,13 @@ __global__ void __launch_bounds__(256) k_generate(const LaunchCtx* __restrict__ 
         c.q.counts[8] = 0u;  // fetch counters of the first extend and shadow stages
         c.q.counts[10] = 0u;
         c.q.counts[12] = 0u; // Q1 mark of the first extend stage
+        c.acc.activeCount[1] = 0; // pixels that go on after the batch (k_accumulate)
     }
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
         initPath<NW>(c, static_cast<uint32_t>(i), jobOffset + static_cast<unsigned long long>(i));
+        if (c.q.nextFlag != nullptr) {
+            c.q.nextFlag[i] = 0; // (a mark that a failed render left)
+        }
     }
 }
 
@@ -1048,12 +1056,13 @@ __device__ __forceinline__ void listMarked(const LaunchCtx& c, int sel)
 // A path whose ray left the scene: previous bounce's NEE, then the
 // environment / background term (PathIntegratorRandCore.h:215-216, 338-346).
 template <int NW>
-__device__ __forceinline__ void shadeMiss(const LaunchCtx& c, uint32_t i, unsigned int* nextCount, uint32_t* nextQueue)
+__device__ __forceinline__ void shadeMiss(const LaunchCtx& c, uint32_t i, bool fresh, unsigned int* nextCount,
+    uint32_t* nextQueue)
 {
     const Waves<NW> wv = pathWaves<NW>(c, i);
     const float4 d4 = c.paths.dir[i];
     const float3 d = f3(d4.x, d4.y, d4.z);
-    const float4 r4 = c.paths.rad[i];
+    const float4 r4 = fresh ? make_float4(0.0f, 0.0f, 0.0f, __int_as_float(0)) : c.paths.rad[i];
     const int depth = __float_as_int(r4.w);
     Col<NW> L;
     const bool sunOn = c.sun.enabled != 0;
@@ -1081,7 +1090,8 @@ __device__ __forceinline__ void shadeMiss(const LaunchCtx& c, uint32_t i, unsign
 }
 
 // Shading of the paths that hit a triangle, then of those that left the scene.
-// One thread per queued path.  (The misses in this launch and not in one of
+// One thread per queued path.  fresh: every path is at depth 0, where the state
+// that initPath leaves out is known.  (The misses in this launch and not in one of
 // their own: they start in the blocks that the hits leave idle, and a bounce of
 // few paths has one launch less: 4 waves of 1024^2 pixels 7.1 -> 6.97 ms with the
 // merged listing pass below.)
@@ -1104,7 +1114,7 @@ constexpr int kShadeThreads = 512;
 #endif
 template <int NW>
 __global__ void __launch_bounds__(kShadeThreads, PT_SHADE_MIN_BLOCKS)
-    k_shade(const LaunchCtx* __restrict__ cp, int sel, int iter)
+    k_shade(const LaunchCtx* __restrict__ cp, int sel, int iter, bool fresh)
 {
     const LaunchCtx& c = *cp;
     const unsigned int count = c.q.counts[5 + 2 * (iter & 1)];
@@ -1129,6 +1139,7 @@ __global__ void __launch_bounds__(kShadeThreads, PT_SHADE_MIN_BLOCKS)
         Ctx cx;
         bool emitterMis = false, misVertex = false;
         bool pendEnv = false, pendEmis = false;
+        bool visEnv = false, visEmis = false; // next-event terms of the previous bounce
         bool cont = false;
         curandStateXORWOW st;
         __syncthreads();
@@ -1136,7 +1147,9 @@ __global__ void __launch_bounds__(kShadeThreads, PT_SHADE_MIN_BLOCKS)
             i = queue[k];
             scene = &sceneOf(c, i);
             wv = pathWaves<NW>(c, i);
-            r4 = c.paths.rad[i];
+            r4 = fresh ? make_float4(0.0f, 0.0f, 0.0f, __int_as_float(0)) : c.paths.rad[i];
+            visEnv = !fresh && c.paths.visEnv[i] != 0;
+            visEmis = !fresh && c.paths.visEmis[i] != 0;
             depth = __float_as_int(r4.w);
             // RGB: the radiance stays in registers through the bounce.  Spectral: it
             // is updated in memory (NEE of the previous bounce and the emission, in
@@ -1146,10 +1159,10 @@ __global__ void __launch_bounds__(kShadeThreads, PT_SHADE_MIN_BLOCKS)
                 L = loadCol<NW>(r4, c.paths.radS, cap, i);
                 // NEE contributions of the previous bounce, in the reference's order
                 // (the flags are clear for a path that starts at this bounce).
-                if (c.paths.visEnv[i]) {
+                if (visEnv) {
                     L = cadd(L, pendingEnv<NW>(c, i));
                 }
-                if (c.paths.visEmis[i]) {
+                if (visEmis) {
                     L = cadd(L, pendingEmis<NW>(c, i));
                 }
             }
@@ -1162,7 +1175,7 @@ __global__ void __launch_bounds__(kShadeThreads, PT_SHADE_MIN_BLOCKS)
             const float4 d4 = c.paths.dir[i];
             d = f3(d4.x, d4.y, d4.z);
             const float4 o4 = c.paths.orig[i];
-            const float4 t4 = c.paths.thr[i];
+            const float4 t4 = fresh ? make_float4(1.0f, 1.0f, 1.0f, 1.0f) : c.paths.thr[i];
             if constexpr (NW == 0) {
                 T = loadCol<NW>(t4, c.paths.thrS, cap, i);
             } else {
@@ -1232,10 +1245,10 @@ __global__ void __launch_bounds__(kShadeThreads, PT_SHADE_MIN_BLOCKS)
                 cx.m.g = 1.0f;
                 cx.m.b = 1.0f;
                 Col<NW> Lm = depth == 0 ? czero<NW>() : loadCol<NW>(r4, c.paths.radS, cap, i);
-                if (c.paths.visEnv[i]) {
+                if (visEnv) {
                     Lm = cadd(Lm, pendingEnv<NW>(c, i));
                 }
-                if (c.paths.visEmis[i]) {
+                if (visEmis) {
                     Lm = cadd(Lm, pendingEmis<NW>(c, i));
                 }
                 // emission (PathIntegratorRandCore.h:248)
@@ -1459,10 +1472,10 @@ __global__ void __launch_bounds__(kShadeThreads, PT_SHADE_MIN_BLOCKS)
                     L = loadCol<NW>(r4, c.paths.radS, cap, i);
                     if (depth >= c.maxDepth) {
                         // (no read-modify-write happened: add the previous bounce's NEE here)
-                        if (c.paths.visEnv[i]) {
+                        if (visEnv) {
                             L = cadd(L, pendingEnv<NW>(c, i));
                         }
-                        if (c.paths.visEmis[i]) {
+                        if (visEmis) {
                             L = cadd(L, pendingEmis<NW>(c, i));
                         }
                     }
@@ -1476,7 +1489,7 @@ __global__ void __launch_bounds__(kShadeThreads, PT_SHADE_MIN_BLOCKS)
     }    const unsigned int misses = c.q.counts[4 + 2 * (iter & 1)];
     for (unsigned int k = (gridDim.x - 1u - blockIdx.x) * blockDim.x + threadIdx.x; k < misses;
          k += gridDim.x * blockDim.x) {
-        shadeMiss<NW>(c, c.q.missQueue[k], nextCount, nextQueue);
+        shadeMiss<NW>(c, c.q.missQueue[k], fresh, nextCount, nextQueue);
     }
 }
 
@@ -1868,14 +1881,15 @@ int shadowLaneInstOccupancy()
 {
     return blocksPerSm(k_shadow_lane<true, false>, kTraceThreads, traceSmemBytes<true>());
 }
-void launchShade(const LaunchCtx* c, int sel, int iter, int grid, int nw, cudaStream_t s)
+void launchShade(const LaunchCtx* c, int sel, int iter, bool first, int grid, int nw, cudaStream_t s)
 {
+    const bool fresh = first && PT_PATH_GENERATIONS != 0;
     if (nw == 8) {
-        k_shade<8><<<grid, kShadeThreads, 0, s>>>(c, sel, iter);
+        k_shade<8><<<grid, kShadeThreads, 0, s>>>(c, sel, iter, fresh);
     } else if (nw == 4) {
-        k_shade<4><<<grid, kShadeThreads, 0, s>>>(c, sel, iter);
+        k_shade<4><<<grid, kShadeThreads, 0, s>>>(c, sel, iter, fresh);
     } else {
-        k_shade<0><<<grid, kShadeThreads, 0, s>>>(c, sel, iter);
+        k_shade<0><<<grid, kShadeThreads, 0, s>>>(c, sel, iter, fresh);
     }
 }
 void launchShadow(const LaunchCtx* c, int iter, int grid, bool count, bool inst, bool lane, bool multi, cudaStream_t s)

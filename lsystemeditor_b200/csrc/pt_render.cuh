@@ -177,7 +177,8 @@ int extendLaneInstOccupancy();
 int shadowLaneInstOccupancy();
 // Resident blocks per SM of the shade kernel for nw wavelengths (0 = RGB).
 int shadeOccupancy(int nw);
-void launchShade(const LaunchCtx* d, int sel, int iter, int grid, int nw, cudaStream_t s);
+// first: the first bounce after launchGenerate.
+void launchShade(const LaunchCtx* d, int sel, int iter, bool first, int grid, int nw, cudaStream_t s);
 // Shadow stage.  lane: per-lane ray replacement (k_shadow_lane; flat scenes,
 // no visit counting), else one warp per 32 queued rays (k_shadow).
 void launchShadow(const LaunchCtx* d, int iter, int grid, bool count, bool inst, bool lane, bool multi, cudaStream_t s);
