@@ -247,6 +247,8 @@ template <int NW> __device__ __forceinline__ void storeCol(float4* rgb, float4* 
         }
     }
 }
+// Depth and medium IOR of a spectral path, in the place of its RGB radiance.
+__device__ __forceinline__ float2* depthEta(const LaunchCtx& c) { return reinterpret_cast<float2*>(c.paths.rad); }
 template <int NW> __device__ __forceinline__ Col<NW> pendingEnv(const LaunchCtx& c, uint32_t i)
 {
     if constexpr (NW == 0) {
@@ -578,7 +580,11 @@ template <int NW> __device__ __forceinline__ void initPath(const LaunchCtx& c, u
     // 329 -> 281 us).
 #if !PT_PATH_GENERATIONS
     c.paths.thr[i] = make_float4(1.0f, 1.0f, 1.0f, 1.0f);
-    c.paths.rad[i] = make_float4(0.0f, 0.0f, 0.0f, __int_as_float(0));
+    if constexpr (NW == 0) {
+        c.paths.rad[i] = make_float4(0.0f, 0.0f, 0.0f, __int_as_float(0));
+    } else {
+        depthEta(c)[i] = make_float2(__int_as_float(0), 1.0f);
+    }
     c.paths.visEnv[i] = 0;
     c.paths.visEmis[i] = 0;
 #endif
@@ -1062,7 +1068,14 @@ __device__ __forceinline__ void shadeMiss(const LaunchCtx& c, uint32_t i, bool f
     const Waves<NW> wv = pathWaves<NW>(c, i);
     const float4 d4 = c.paths.dir[i];
     const float3 d = f3(d4.x, d4.y, d4.z);
-    const float4 r4 = fresh ? make_float4(0.0f, 0.0f, 0.0f, __int_as_float(0)) : c.paths.rad[i];
+    float4 r4 = make_float4(0.0f, 0.0f, 0.0f, __int_as_float(0));
+    if (!fresh) {
+        if constexpr (NW == 0) {
+            r4 = c.paths.rad[i];
+        } else {
+            r4.w = depthEta(c)[i].x;
+        }
+    }
     const int depth = __float_as_int(r4.w);
     Col<NW> L;
     const bool sunOn = c.sun.enabled != 0;
@@ -1078,7 +1091,7 @@ __device__ __forceinline__ void shadeMiss(const LaunchCtx& c, uint32_t i, bool f
             L = cadd(L, pendingEmis<NW>(c, i));
         }
         if (!black) {
-            const Col<NW> T = loadCol<NW>(c.paths.thr[i], c.paths.thrS, c.paths.capacity, i);
+            const Col<NW> T = loadCol<NW>(NW == 0 ? c.paths.thr[i] : r4, c.paths.thrS, c.paths.capacity, i);
             const Col<NW> Le = sunOn ? skyCol<NW>(c, d, wv) : envCol<NW>(c, d, wv);
             const float lp = sunOn ? skyPdf(c, d) : envPdf(c.env, d);
             const float w = misBalance(fabsf(d4.w), lp);
@@ -1123,6 +1136,7 @@ __global__ void __launch_bounds__(kShadeThreads, PT_SHADE_MIN_BLOCKS)
     uint32_t* nextQueue = c.q.extend[sel ^ 1];
     const int debugFlags = c.params.brdf_debug_flags;
     const int cap = c.paths.capacity;
+    __shared__ float4 sRad[NW == 0 ? 1 : NW / 4][kShadeThreads]; // a thread's own column
     // (the whole block runs the loop: barriers)
     for (unsigned int base = blockIdx.x * blockDim.x; base < count; base += gridDim.x * blockDim.x) {
         const unsigned int k = base + threadIdx.x;
@@ -1147,13 +1161,22 @@ __global__ void __launch_bounds__(kShadeThreads, PT_SHADE_MIN_BLOCKS)
             i = queue[k];
             scene = &sceneOf(c, i);
             wv = pathWaves<NW>(c, i);
-            r4 = fresh ? make_float4(0.0f, 0.0f, 0.0f, __int_as_float(0)) : c.paths.rad[i];
+            r4 = make_float4(0.0f, 0.0f, 0.0f, __int_as_float(0));
+            if (!fresh) {
+                if constexpr (NW == 0) {
+                    r4 = c.paths.rad[i];
+                } else {
+                    const float2 de = depthEta(c)[i];
+                    r4.w = de.x;
+                    eta = de.y;
+                }
+            }
             visEnv = !fresh && c.paths.visEnv[i] != 0;
             visEmis = !fresh && c.paths.visEmis[i] != 0;
             depth = __float_as_int(r4.w);
             // RGB: the radiance stays in registers through the bounce.  Spectral: it
-            // is updated in memory (NEE of the previous bounce and the emission, in
-            // one read-modify-write below) and reloaded only by a path that ends.
+            // waits in shared memory once the NEE of the previous bounce and the
+            // emission are added.
             L = czero<NW>();
             if constexpr (NW == 0) {
                 L = loadCol<NW>(r4, c.paths.radS, cap, i);
@@ -1175,7 +1198,7 @@ __global__ void __launch_bounds__(kShadeThreads, PT_SHADE_MIN_BLOCKS)
             const float4 d4 = c.paths.dir[i];
             d = f3(d4.x, d4.y, d4.z);
             const float4 o4 = c.paths.orig[i];
-            const float4 t4 = fresh ? make_float4(1.0f, 1.0f, 1.0f, 1.0f) : c.paths.thr[i];
+            const float4 t4 = fresh ? make_float4(1.0f, 1.0f, 1.0f, 1.0f) : NW == 0 ? c.paths.thr[i] : make_float4(1.0f, 1.0f, 1.0f, eta);
             if constexpr (NW == 0) {
                 T = loadCol<NW>(t4, c.paths.thrS, cap, i);
             } else {
@@ -1256,7 +1279,7 @@ __global__ void __launch_bounds__(kShadeThreads, PT_SHADE_MIN_BLOCKS)
                 for (int q = 0; q < NW; ++q) {
                     Lm.v[q] = Lm.v[q] + T.v[q] * (rho.v[q] * emission);
                 }
-                storeCol<NW>(nullptr, c.paths.radS, cap, i, Lm, 0.0f);
+                storeCol<NW>(nullptr, &sRad[0][threadIdx.x], kShadeThreads, 0u, Lm, 0.0f);
             }
             rngLoad(c.paths, i, st);
         }
@@ -1436,7 +1459,7 @@ __global__ void __launch_bounds__(kShadeThreads, PT_SHADE_MIN_BLOCKS)
                             dot3(n, smp.dir) > 0.0f && !inTransmitCones(cx, smp.dir);
                         c.paths.dir[i] = make_float4(smp.dir.x, smp.dir.y, smp.dir.z,
                             (emitterMis && !misSample) ? -smp.pdf : smp.pdf);
-                        storeCol<NW>(c.paths.thr, c.paths.thrS, cap, i, T, eta);
+                        storeCol<NW>(NW == 0 ? c.paths.thr : nullptr, c.paths.thrS, cap, i, T, eta);
                         cont = true;
                     }
                 }
@@ -1459,9 +1482,20 @@ __global__ void __launch_bounds__(kShadeThreads, PT_SHADE_MIN_BLOCKS)
                     recyclePath<NW>(c, i, nextCount, nextQueue);
                 }
             } else {
+                if (live) {
+                    L = loadCol<NW>(r4, &sRad[0][threadIdx.x], kShadeThreads, 0u);
+                } else {
+                    L = loadCol<NW>(r4, c.paths.radS, cap, i);
+                    if (visEnv) {
+                        L = cadd(L, pendingEnv<NW>(c, i));
+                    }
+                    if (visEmis) {
+                        L = cadd(L, pendingEmis<NW>(c, i));
+                    }
+                }
                 if (cont || pendEnv || pendEmis) {
-                    // the radiance is in radS already
-                    c.paths.rad[i] = make_float4(0.0f, 0.0f, 0.0f, __int_as_float(cont ? depth + 1 : depth));
+                    storeCol<NW>(nullptr, c.paths.radS, cap, i, L, 0.0f);
+                    depthEta(c)[i] = make_float2(__int_as_float(cont ? depth + 1 : depth), eta);
                     if (cont) {
                         queueNext(c, i, nextCount, nextQueue);
                     } else {
@@ -1469,16 +1503,6 @@ __global__ void __launch_bounds__(kShadeThreads, PT_SHADE_MIN_BLOCKS)
                         c.q.finish[s] = i;
                     }
                 } else {
-                    L = loadCol<NW>(r4, c.paths.radS, cap, i);
-                    if (depth >= c.maxDepth) {
-                        // (no read-modify-write happened: add the previous bounce's NEE here)
-                        if (visEnv) {
-                            L = cadd(L, pendingEnv<NW>(c, i));
-                        }
-                        if (visEmis) {
-                            L = cadd(L, pendingEmis<NW>(c, i));
-                        }
-                    }
                     writeSample<NW>(c, i, L, wv);
                     recyclePath<NW>(c, i, nextCount, nextQueue);
                 }
@@ -1486,7 +1510,8 @@ __global__ void __launch_bounds__(kShadeThreads, PT_SHADE_MIN_BLOCKS)
                 c.paths.visEmis[i] = 0;
             }
         }
-    }    const unsigned int misses = c.q.counts[4 + 2 * (iter & 1)];
+    }
+    const unsigned int misses = c.q.counts[4 + 2 * (iter & 1)];
     for (unsigned int k = (gridDim.x - 1u - blockIdx.x) * blockDim.x + threadIdx.x; k < misses;
          k += gridDim.x * blockDim.x) {
         shadeMiss<NW>(c, c.q.missQueue[k], fresh, nextCount, nextQueue);

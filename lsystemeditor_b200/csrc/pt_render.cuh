@@ -35,8 +35,8 @@ struct PathSoA {
     uint16_t* scene = nullptr;   // scene of the path (written only when more than one scene is rendered)
     // spectral mode (NW wavelengths per path): the path's hero draw, and NW / 4
     // float4 per path of throughput, radiance and pending NEE contributions,
-    // word j of path i at [j * capacity + i] (the RGB fields above then carry
-    // only the medium IOR in thr.w and the depth in rad.w)
+    // word j of path i at [j * capacity + i] (of the RGB fields above only rad is
+    // then used, for a float2 of depth and medium IOR per path)
     float* hero = nullptr;
     float4* thrS = nullptr;
     float4* radS = nullptr;
