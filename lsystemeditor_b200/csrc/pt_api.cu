@@ -209,7 +209,7 @@ struct pt_renderer {
     DevBuf<float4> previewBuf;            // all levels, coarsest first
     DevBuf<char> queryBuf;                // inputs and results of pt_trace_rays
     std::unique_ptr<HostCopier> copier;   // staged copies from and to pageable memory
-    cudaStream_t copyStream = nullptr;    // uploads beside the work on `stream`
+    cudaStream_t copyStream = nullptr;    // uploads beside the work on `stream` (made by the first large mesh)
     cudaEvent_t copyEvent = nullptr;      // orders the two
     // region render (PathTracer.h:134-140)
     bool regionEnabled = false;
@@ -243,11 +243,11 @@ struct pt_renderer {
     // shadow nodes and tris), traversal stack overflows (32 bits)
     DevBuf<unsigned long long> qStats;
     int gridExtend = 0, gridShade = 0, gridShadow = 0;
-    int gridExtendLane = 0;          // grid of the per-lane closest-hit kernel
-    int gridShadowLane = 0;          // grid of the per-lane shadow kernel
-    int gridExtendLaneInst = 0;      // grids of the per-lane kernels of instanced scenes
+    int gridExtendLane = 0;          // grid of the whole-warp closest-hit kernel
+    int gridShadowLane = 0;          // grid of the whole-warp shadow kernel
+    int gridExtendLaneInst = 0;      // grids of the whole-warp kernels of instanced scenes
     int gridShadowLaneInst = 0;
-    bool extendLane = false;         // per-lane ray replacement in this render's closest-hit stage
+    bool extendLane = false;         // whole-warp traversal in this render
     int extendMode = PT_EXTEND_MODE_AUTO;
     // CUDA graphs of four bounce iterations (the first block of a batch, later
     // blocks) and the launch configuration they were captured for
@@ -394,9 +394,8 @@ int ensurePaths(pt_renderer* r, int capacity)
 #define PT_SLOT_ORDER 1
 #endif
 
-// Slot-ordered next queue (k_next_queue): with the per-lane closest-hit kernel,
-// whose queue order does not matter to it, the shade kernels read consecutive
-// slots' path state.
+// Slot-ordered next queue: with the whole-warp traversal, whose queue order does
+// not matter to it, the shade kernels read consecutive slots' path state.
 bool slotOrdered(const pt_renderer* r) { return PT_SLOT_ORDER && r->extendLane; }
 
 LaunchCtx makeCtx(pt_renderer* r)
@@ -1024,27 +1023,42 @@ int setSceneMesh(pt_renderer* r, SceneSlot& sl, const pt_mesh* mesh)
             return st;
         }
     }
+    bool beside = false;
     if (n > 0) {
         if (!sl.positions.ensure(9ull * n) || !r->stage.ensure(15ull * n) || !r->stageIds.ensure(n)) {
             return fail(r, PT_ERR_OUT_OF_MEMORY, "mesh upload failed for %u triangles", n);
         }
-        // the build starts with the positions and ids; the normals and uvs are
-        // uploaded beside it
+        // the build starts with the positions and ids; the normals and uvs of a
+        // large mesh are uploaded beside it
         const HostCopier::Piece first[2] = {{sl.positions.p, const_cast<float*>(mesh->positions), 9ull * n * sizeof(float)},
             {r->stageIds.p, const_cast<uint32_t*>(mesh->material_ids), n * sizeof(uint32_t)}};
         const HostCopier::Piece second[2] = {{r->stage.p, const_cast<float*>(mesh->normals), 9ull * n * sizeof(float)},
             {r->stage.p + 9ull * n, const_cast<float*>(mesh->uvs), 6ull * n * sizeof(float)}};
-        PT_CHECK(r, cudaEventRecord(r->copyEvent, s));
-        PT_CHECK(r, cudaStreamWaitEvent(r->copyStream, r->copyEvent, 0));
+        beside = HostCopier::large(second, 2);
+        if (beside) {
+            if (r->copyStream == nullptr) {
+                PT_CHECK(r, cudaStreamCreateWithFlags(&r->copyStream, cudaStreamNonBlocking));
+            }
+            if (r->copyEvent == nullptr) {
+                PT_CHECK(r, cudaEventCreateWithFlags(&r->copyEvent, cudaEventDisableTiming));
+            }
+            PT_CHECK(r, cudaEventRecord(r->copyEvent, s));
+            PT_CHECK(r, cudaStreamWaitEvent(r->copyStream, r->copyEvent, 0));
+        }
         PT_CHECK(r, r->copier->beginUpload(first, 2, s));
         PT_CHECK(r, r->copier->finish());
-        PT_CHECK(r, r->copier->beginUpload(second, 2, r->copyStream));
+        PT_CHECK(r, r->copier->beginUpload(second, 2, beside ? r->copyStream : s));
+        if (!beside) {
+            PT_CHECK(r, r->copier->finish());
+        }
     }
     {
-        const int st = finishScene(r, sl, n, n > 0);
+        const int st = finishScene(r, sl, n, beside);
         if (st != PT_OK) {
-            r->copier->finish(); // (the caller's arrays are not read after the call)
-            cudaStreamSynchronize(r->copyStream);
+            if (beside) {
+                r->copier->finish(); // (the caller's arrays are not read after the call)
+                cudaStreamSynchronize(r->copyStream);
+            }
             return st;
         }
     }
@@ -1253,7 +1267,7 @@ void releaseBounceGraphs(pt_renderer* r)
     }
 }
 
-// Grid of the closest-hit stage: the per-lane kernel has its own occupancy.
+// Grid of the closest-hit stage: the whole-warp kernel has its own occupancy.
 int extendGrid(const pt_renderer* r, bool count, bool inst)
 {
     if (r->extendLane && !count) {
@@ -1354,8 +1368,6 @@ int pt_create(pt_renderer** out, int device)
     }
     if (cudaSetDevice(r->device) != cudaSuccess ||
         cudaStreamCreateWithFlags(&r->ownStream, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaStreamCreateWithFlags(&r->copyStream, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaEventCreateWithFlags(&r->copyEvent, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreate(&r->ev0) != cudaSuccess || cudaEventCreate(&r->ev1) != cudaSuccess) {
         delete r;
         return PT_ERR_CUDA;

@@ -50,6 +50,16 @@ public:
         release();
     }
 
+    // Worth staging on its first occurrence.
+    static bool large(const Piece* p, size_t n)
+    {
+        size_t total = 0;
+        for (size_t i = 0; i < n; ++i) {
+            total += p[i].bytes;
+        }
+        return total >= kAtOnceBytes;
+    }
+
     // Starts copying the pieces to the device on stream s; the sources may be
     // changed, and work that reads the copies be put on s, after finish().
     // Transfers too small to gain, from memory that is not pageable or on a

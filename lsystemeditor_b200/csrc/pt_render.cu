@@ -7,20 +7,18 @@
 //
 //   generate   camera ray per (pixel, sample): curand_init with the reference
 //              seed, jitter + lens draws (PathTracer.cu:69-96)
-//   extend     closest hit for every live path            (pt_trace.cuh);
-//              large flat scenes: per-lane ray replacement (k_extend_lane)
-//              + k_route, which splits the queue into miss and hit queues
+//   extend     closest hit for every live path (pt_traverse.cuh), then k_route,
+//              which splits the queue into miss and hit queues
 //   shade      pending NEE resolve, miss/env MIS, emission, environment and
 //              emissive NEE (shadow rays queued), BSDF sample, throughput,
 //              subsurface tier B, Russian roulette, continuation ray
 //   shadow     any-hit occlusion for the queued shadow rays
-//   finalize   paths that ended with shadow rays in flight
-//   next_queue (with k_extend_lane) the next bounce's extend queue in slot
-//              order, from the slots the shade kernels marked
+//   finalize   paths that ended with shadow rays in flight; the next bounce's
+//              extend queue in slot order, from the slots the shade kernel marked
 //   accumulate per pixel, the batch's samples in sample order: running mean,
 //              Welford luminance variance, convergence every 4 samples
 //              (PathTracer.cu:232-272)
-//   compact    active-pixel list without converged pixels
+//   compact    active-pixel list without converged pixels, where it changed
 //
 // Radiance is added in exactly the reference's order: emission, env NEE,
 // emissive NEE (resolved after the shadow stage), then at the next bounce the
@@ -593,7 +591,7 @@ template <int NW> __device__ __forceinline__ void initPath(const LaunchCtx& c, u
     }
 }
 
-// Path i joins the next bounce's extend queue: marked for k_next_queue in
+// Path i joins the next bounce's extend queue: marked for listMarked in
 // slot-ordered mode, else pushed (one atomic per warp).
 __device__ __forceinline__ void queueNext(const LaunchCtx& c, uint32_t i, unsigned int* nextCount, uint32_t* nextQueue)
 {

@@ -58,7 +58,7 @@ struct BatchInfo {
 struct QueueSet {
     uint32_t* extend[2] = {nullptr, nullptr}; // path indices, ping-pong
     // slot-ordered mode (non-null): the shade kernels mark the paths of the next
-    // bounce here and k_next_queue lists them in slot order
+    // bounce here and the finalize launch lists them in slot order
     uint8_t* nextFlag = nullptr;
     uint32_t* finish = nullptr;               // paths that ended with shadow rays in flight
     uint32_t* missQueue = nullptr;            // paths whose last ray left the scene
@@ -164,13 +164,13 @@ struct LaunchCtx {
 void launchGenerate(const LaunchCtx* d, int count, int extendSel, int nw, cudaStream_t s,
     unsigned long long jobOffset = 0);
 // inst: compile-time instanced-scene traversal (any scene of the context instanced).
-// Closest-hit stage.  lane: per-lane ray replacement (k_extend_lane + k_route;
-// flat scenes, no visit counting), else one warp-fetch k_extend.
+// Closest-hit stage.  lane: whole-warp traversal (k_extend_lane + k_route; no
+// visit counting), else one ray per lane (k_extend).
 void launchExtend(const LaunchCtx* d, int sel, bool identity, int iter, int grid, bool count, bool inst, bool lane,
     bool multi, cudaStream_t s);
 // Kernels one launchExtend call launches (closest hit, and the routing pass after it).
 int extendKernels(bool count, bool inst, bool lane);
-// Resident blocks per SM of the per-lane kernels.
+// Resident blocks per SM of the whole-warp kernels.
 int extendLaneOccupancy();
 int shadowLaneOccupancy();
 int extendLaneInstOccupancy();
@@ -179,8 +179,8 @@ int shadowLaneInstOccupancy();
 int shadeOccupancy(int nw);
 // first: the first bounce after launchGenerate.
 void launchShade(const LaunchCtx* d, int sel, int iter, bool first, int grid, int nw, cudaStream_t s);
-// Shadow stage.  lane: per-lane ray replacement (k_shadow_lane; flat scenes,
-// no visit counting), else one warp per 32 queued rays (k_shadow).
+// Shadow stage.  lane: whole-warp traversal (k_shadow_lane; no visit counting),
+// else one ray per lane (k_shadow).
 void launchShadow(const LaunchCtx* d, int iter, int grid, bool count, bool inst, bool lane, bool multi, cudaStream_t s);
 // list: slot-ordered mode, the next bounce's extend queue from the marked slots.
 void launchFinalize(const LaunchCtx* d, int sel, int grid, int nw, bool list, cudaStream_t s);

@@ -21,15 +21,16 @@
 // Why: in a free-running loop (a lane fetched and stepped on its own) 6 of 32
 // lanes worked per executed instruction, a node's triangles were tested one
 // after the other, and every finished ray was an atomic on one address.  It is
-// bound by the latency of the node and triangle loads and by issue (16 of 32
-// lanes, 45% of the issue slots; DRAM idles, the scene is in L2).  Registers
+// bound by issue and by the latency of the node and triangle loads (20 of 32
+// lanes, 64 - 68% of the issue slots, the ALU pipe at 53 - 59%; DRAM idles, the
+// scene is in L2).  Registers
 // matter more than warps: with spills at 64 registers it lost a quarter, so the
 // per-ray words that only the ends of a ray need are in shared memory, and
 // rays of quirk Q1 are traced elsewhere (their call costs registers here).
-// Measured: closest hit of the large frame (972k triangles, 402M rays) 159.9 ->
-// 85.4 ms, of one 1024^2 wave (1.6M rays over 8 launches) 1.86 -> 0.95 ms (1.34
-// without stealing: the launches of late bounces wait for their longest ray),
-// shadow rays of a 513x511 32-spp emitter-MIS frame 3.73 -> 2.10 ms.
+// Measured: closest hit of the large frame (972k triangles, 402M rays) 163 ->
+// 80 ms, of one 1024^2 wave (1.6M rays over 8 launches) 1.86 -> 0.77 ms (without
+// stealing a third more: the launches of late bounces wait for their longest
+// ray), shadow rays of a 513x511 32-spp emitter-MIS frame 3.73 -> 2.0 ms.
 #pragma once
 
 #include "pt_trace.cuh"
