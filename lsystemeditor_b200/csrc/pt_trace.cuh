@@ -174,6 +174,27 @@ __device__ __forceinline__ Pair2 fma2(Pair2 a, Pair2 b, Pair2 c)
     return r;
 }
 
+// A bound on how far the t of a box's near plane may lie above the t of a
+// triangle in the box, by rounding alone: q a + b is off by a few ulps of
+// |b| = |p - o| |1/d| and not of t, and the t of a triangle by ulps of its
+// vertices' distance over |d . n|.  Near a surface both are far more than
+// kSlabWiden of t, so of two hits closer together than this a ray may return
+// either, depending on which it tests first.  16 ulps (1 is enough in 200 scenes
+// of overlapping coplanar rectangles) of the farthest distance to the tree's box
+// times the largest |1/d|, capped: a plane that the ray is nearly parallel to is
+// hardly ever the near one.
+__device__ __forceinline__ float hitSlack(const CwNode* __restrict__ nodes, float3 o, float3 idir)
+{
+    const uint4 w = __ldg(reinterpret_cast<const uint4*>(nodes));
+    const float ex = __uint_as_float((w.w & 0xffu) << 23), ey = __uint_as_float(((w.w >> 8) & 0xffu) << 23),
+                ez = __uint_as_float(((w.w >> 16) & 0xffu) << 23);
+    const float far = fmaxf(fmaxf(fmaf(255.0f, ex, fabsf(__uint_as_float(w.x) - o.x)),
+                                fmaf(255.0f, ey, fabsf(__uint_as_float(w.y) - o.y))),
+        fmaf(255.0f, ez, fabsf(__uint_as_float(w.z) - o.z)));
+    const float steep = fminf(fmaxf(fmaxf(fabsf(idir.x), fabsf(idir.y)), fabsf(idir.z)), 65536.0f);
+    return 16.0f * 5.9604645e-8f * far * steep;
+}
+
 // Intersects the ray with the eight quantised child boxes of a node.
 // Returns the hit mask: bits 24..31 internal children (slot ^ octinv), bits
 // 0..23 leaf triangles (node-local offsets).
