@@ -208,7 +208,7 @@ struct pt_renderer {
     int previewDone = -1;                 // finest preview level rendered since the last reset
     DevBuf<float4> previewBuf;            // all levels, coarsest first
     DevBuf<char> queryBuf;                // inputs and results of pt_trace_rays
-    std::unique_ptr<HostCopier> copier;   // staged copies from and to pageable memory
+    HostCopier::Owner copier;             // staged copies from and to pageable memory
     cudaStream_t copyStream = nullptr;    // uploads beside the work on `stream` (made by the first large mesh)
     cudaEvent_t copyEvent = nullptr;      // orders the two
     // region render (PathTracer.h:134-140)

@@ -11,6 +11,9 @@
 //
 // One copier belongs to one renderer: the threads, 8 MB of pinned memory and
 // the events are made when its transfers are worth it and given back with it.
+// A process forked off has none of the threads: there the copier copies plainly
+// and is left alone when its owner goes (a condition variable that vanished
+// threads wait on cannot be destroyed).
 #pragma once
 
 #include <cuda_runtime.h>
@@ -19,9 +22,12 @@
 #include <atomic>
 #include <condition_variable>
 #include <cstring>
+#include <memory>
 #include <mutex>
 #include <thread>
 #include <vector>
+
+#include <unistd.h>
 
 namespace pt {
 
@@ -32,6 +38,16 @@ public:
         void* host; // (only read by uploads)
         size_t bytes;
     };
+
+    struct Deleter {
+        void operator()(HostCopier* c) const
+        {
+            if (!c->forked()) {
+                delete c;
+            }
+        }
+    };
+    using Owner = std::unique_ptr<HostCopier, Deleter>;
 
     explicit HostCopier(int device) : device_(device) {}
     HostCopier(const HostCopier&) = delete;
@@ -71,7 +87,7 @@ public:
 
     cudaError_t finish()
     {
-        if (!running_) {
+        if (!running_ || forked()) {
             return cudaSuccess;
         }
         work(0);
@@ -93,11 +109,13 @@ private:
     static constexpr size_t kAtOnceBytes = 32u << 20;
     static constexpr int kBefore = 4;
 
+    bool forked() const { return getpid() != process_; }
+
     cudaError_t begin(const Piece* p, size_t n, cudaStream_t s, bool up)
     {
         cudaError_t e = finish();
         size_t total = 0;
-        bool staged = s != cudaStreamPerThread;
+        bool staged = s != cudaStreamPerThread && !forked();
         for (size_t i = 0; i < n && e == cudaSuccess; ++i) {
             total += p[i].bytes;
             cudaPointerAttributes a{};
@@ -277,6 +295,7 @@ private:
     }
 
     const int device_;
+    const pid_t process_ = getpid();
     int state_ = 0; // 0 not tried, 1 ready, -1 not available
     int small_ = 0; // transfers from kMinBytes to kAtOnceBytes so far
     char* pinned_ = nullptr;
