@@ -6,8 +6,8 @@
 // Each worker copies its own slices into its own pinned buffers and enqueues
 // them itself, so workers meet only at the start and the end of a transfer.
 // Measured: opening a 972k-triangle mesh (97 MB; the shading half beside the BVH
-// build) 11.6 -> 4.5 ms, 200k ray queries (6.4 MB in, 5.8 MB out) 1.90 -> 1.55 ms;
-// a 3 MB image gradient, still in the caller's cache, 0.5 ms slower.
+// build) 11.6 -> 4.5 ms, 1M ray queries (32 MB in, 29 MB out) 8.2 -> 5.0 ms; a 3 MB
+// image gradient, still in the caller's cache, 0.5 ms slower.
 //
 // One copier belongs to one renderer: the threads, 8 MB of pinned memory and
 // the events are made when its transfers are worth it and given back with it.
@@ -66,14 +66,14 @@ public:
         release();
     }
 
-    // Worth staging on its first occurrence.
+    // Worth a stream of its own beside other work.
     static bool large(const Piece* p, size_t n)
     {
         size_t total = 0;
         for (size_t i = 0; i < n; ++i) {
             total += p[i].bytes;
         }
-        return total >= kAtOnceBytes;
+        return total >= kBesideBytes;
     }
 
     // Starts copying the pieces to the device on stream s; the sources may be
@@ -101,13 +101,15 @@ private:
     static constexpr size_t kSlice = 1024u << 10; // (256 KB: 5.8 ms for the mesh above, 512: 4.8, 1024: 4.5)
     static constexpr int kWorkers = 4; // the calling thread is one of them
     static constexpr int kBuffers = 2; // per worker: one is filled while the other is in flight
-    // Below kMinBytes the wake-up of the workers costs more than they save.
-    // Making the pinned memory takes 1 - 5 ms, what a transfer of kAtOnceBytes
-    // or a few dozen of the smallest gain back: smaller ones are staged from the
-    // fifth on (a renderer that is asked a few queries makes none).
-    static constexpr size_t kMinBytes = 4u << 20;
-    static constexpr size_t kAtOnceBytes = 32u << 20;
-    static constexpr int kBefore = 4;
+    // Staging gains from about 12 MB on (plain, staged: 131k-ray queries, 4 MB in
+    // and out, 1.15, 1.15 ms; 200k 1.8, 1.9; 500k, 16 and 14 MB, 4.05, 3.07; 1M 8.2,
+    // 5.0; meshes of 150k triangles, 6 + 9 MB, 1.48, 1.63; 300k, 12 + 18 MB, 2.4, 2.1).
+    static constexpr size_t kMinBytes = 12u << 20;
+    // The pinned memory and the threads take 4 - 8 ms to make, what staging gains on
+    // about this much: made once that much has been copied plainly, so that few
+    // transfers never pay for it and many pay once.
+    static constexpr size_t kWorthBytes = 96u << 20;
+    static constexpr size_t kBesideBytes = 32u << 20;
 
     bool forked() const { return getpid() != process_; }
 
@@ -126,9 +128,13 @@ private:
             }
         }
         cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-        if (staged && total >= kMinBytes && cudaStreamIsCapturing(s, &cs) == cudaSuccess &&
-            cs == cudaStreamCaptureStatusNone && e == cudaSuccess &&
-            (total >= kAtOnceBytes || state_ > 0 || ++small_ > kBefore) && ready()) {
+        staged = staged && total >= kMinBytes && cudaStreamIsCapturing(s, &cs) == cudaSuccess &&
+            cs == cudaStreamCaptureStatusNone && e == cudaSuccess;
+        if (staged && plain_ < kWorthBytes) {
+            plain_ += total;
+            staged = false;
+        }
+        if (staged && ready()) {
             pieces_.assign(p, p + n);
             stream_ = s;
             up_ = up;
@@ -297,7 +303,7 @@ private:
     const int device_;
     const pid_t process_ = getpid();
     int state_ = 0; // 0 not tried, 1 ready, -1 not available
-    int small_ = 0; // transfers from kMinBytes to kAtOnceBytes so far
+    size_t plain_ = 0; // bytes copied plainly that could have been staged (up to kWorthBytes and a transfer)
     char* pinned_ = nullptr;
     cudaEvent_t events_[kBuffers * kWorkers] = {};
     std::vector<std::thread> threads_;

@@ -54,6 +54,35 @@ HostCopier::Owner warm()
     return c;
 }
 
+// The pinned memory is made once 96 MB of transfers of at least 12 MB have been
+// copied plainly: few or small transfers never pay for it.
+void stagingRule()
+{
+    HostCopier::Owner c(new HostCopier(0));
+    auto moves = [&](size_t n, int times, bool up) {
+        std::vector<char> a = bytes(n, static_cast<uint32_t>(n)), b(n);
+        for (int k = 0; k < times; ++k) {
+            std::fill(b.begin(), b.end(), 0);
+            CHECK(move(*c, a, b, up) == cudaSuccess && a == b);
+        }
+    };
+    moves(12 * kMb - 1, 40, true);
+    moves(1, 3, false);
+    CHECK(fake::hostAllocs == 0);
+    moves(12 * kMb, 4, true);
+    moves(12 * kMb, 4, false);
+    CHECK(fake::hostAllocs == 0);
+    const int before = fake::copies;
+    moves(12 * kMb + 1, 1, true); // (13 slices)
+    CHECK(fake::hostAllocs == 1 && fake::copies == before + 13);
+    moves(12 * kMb - 1, 1, true);
+    CHECK(fake::copies == before + 14);
+    moves(40 * kMb + 77, 3, false);
+    CHECK(fake::hostAllocs == 1 && fake::copies == before + 14 + 3 * 41);
+    c.reset();
+    CHECK(fake::hostFrees == 1);
+}
+
 // A forked child gives the copier back without its threads, and copies plainly.
 void forkedChild()
 {
@@ -84,6 +113,8 @@ int main(int argc, char** argv)
         const std::string name = argv[k];
         if (name == "forked_child") {
             forkedChild();
+        } else if (name == "staging_rule") {
+            stagingRule();
         } else {
             std::printf("no check named %s\n", name.c_str());
             ++failures;
