@@ -45,6 +45,7 @@ template <class T> struct DevBuf {
             count = 1;
         }
         if (cudaMalloc(&p, count * sizeof(T)) != cudaSuccess) {
+            cudaGetLastError(); // (the caller reports it; the next call's launch checks must not find it)
             p = nullptr;
             n = 0;
             return false;

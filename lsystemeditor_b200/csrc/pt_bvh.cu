@@ -924,6 +924,7 @@ int buildBvh(const float* dPositions, uint32_t n, BvhBuffers& out, cudaStream_t 
     const int N = static_cast<int>(n);
     const int nodesBin = 2 * N - 1;
     DeviceArena& ar = out.scratch;
+    ar.failed = false;
     float4* triLo = ar.get<float4>(0, n);
     float4* triHi = ar.get<float4>(1, n);
     unsigned int* cbounds = ar.get<unsigned int>(2, 8);

@@ -14,7 +14,7 @@ struct DeviceArena {
     static constexpr int kSlots = 24;
     void* ptr[kSlots] = {};
     size_t bytes[kSlots] = {};
-    bool failed = false;
+    bool failed = false; // an allocation of the current build failed
 
     void* getBytes(int slot, size_t n)
     {
@@ -28,6 +28,7 @@ struct DeviceArena {
                 bytes[slot] = 0;
             }
             if (cudaMalloc(&ptr[slot], n) != cudaSuccess) {
+                cudaGetLastError(); // (reported through ok())
                 ptr[slot] = nullptr;
                 failed = true;
                 return nullptr;
@@ -98,6 +99,7 @@ struct BvhBuffers {
             nodes = nullptr;
             nodeCapacity = 0;
             if (cudaMalloc(&nodes, n * sizeof(CwNode)) != cudaSuccess) {
+                cudaGetLastError();
                 nodes = nullptr;
                 return false;
             }
@@ -110,6 +112,7 @@ struct BvhBuffers {
             tris = nullptr;
             triCapacity = 0;
             if (cudaMalloc(&tris, t * sizeof(TriVerts)) != cudaSuccess) {
+                cudaGetLastError();
                 tris = nullptr;
                 return false;
             }
