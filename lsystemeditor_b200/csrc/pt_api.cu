@@ -209,7 +209,7 @@ struct pt_renderer {
     int previewDone = -1;                 // finest preview level rendered since the last reset
     DevBuf<float4> previewBuf;            // all levels, coarsest first
     DevBuf<char> queryBuf;                // inputs and results of pt_trace_rays
-    HostCopier::Owner copier;             // staged copies from and to pageable memory
+    std::shared_ptr<HostCopier> copier;   // staged copies from and to pageable memory (the device's)
     cudaStream_t copyStream = nullptr;    // uploads beside the work on `stream` (made by the first large mesh)
     cudaEvent_t copyEvent = nullptr;      // orders the two
     // region render (PathTracer.h:134-140)
@@ -958,7 +958,7 @@ int buildEmissive(pt_renderer* r, SceneSlot& sl, uint32_t n)
 // emissive list and CDF, and the BVH, all on the device.
 // uploading: the normals and uvs are on their way on copyStream; the shading
 // records, which nothing else of the build reads, then come last.
-int finishScene(pt_renderer* r, SceneSlot& sl, uint32_t n, bool uploading = false)
+int finishScene(pt_renderer* r, SceneSlot& sl, uint32_t n, HostCopier::Transfer* uploading = nullptr)
 {
     cudaStream_t s = r->stream;
     sl.triCount = n;
@@ -974,7 +974,7 @@ int finishScene(pt_renderer* r, SceneSlot& sl, uint32_t n, bool uploading = fals
     if (!sl.shade.ensure(n)) {
         return fail(r, PT_ERR_OUT_OF_MEMORY, "shading records allocation failed for %u triangles", n);
     }
-    if (!uploading) {
+    if (uploading == nullptr) {
         launchBuildShade(r->stage.p, r->stage.p + 9ull * n, r->stageIds.p, n, sl.shade.p, s);
         PT_CHECK(r, cudaGetLastError());
     }
@@ -989,8 +989,8 @@ int finishScene(pt_renderer* r, SceneSlot& sl, uint32_t n, bool uploading = fals
     if (st != PT_OK) {
         return fail(r, st, "BVH build: %s", err);
     }
-    if (uploading) {
-        PT_CHECK(r, r->copier->finish());
+    if (uploading != nullptr) {
+        PT_CHECK(r, uploading->finish());
         PT_CHECK(r, cudaEventRecord(r->copyEvent, r->copyStream));
         PT_CHECK(r, cudaStreamWaitEvent(s, r->copyEvent, 0));
         launchBuildShade(r->stage.p, r->stage.p + 9ull * n, r->stageIds.p, n, sl.shade.p, s);
@@ -1025,6 +1025,7 @@ int setSceneMesh(pt_renderer* r, SceneSlot& sl, const pt_mesh* mesh)
         }
     }
     bool beside = false;
+    HostCopier::Transfer uploading(*r->copier);
     if (n > 0) {
         if (!sl.positions.ensure(9ull * n) || !r->stage.ensure(15ull * n) || !r->stageIds.ensure(n)) {
             return fail(r, PT_ERR_OUT_OF_MEMORY, "mesh upload failed for %u triangles", n);
@@ -1046,18 +1047,18 @@ int setSceneMesh(pt_renderer* r, SceneSlot& sl, const pt_mesh* mesh)
             PT_CHECK(r, cudaEventRecord(r->copyEvent, s));
             PT_CHECK(r, cudaStreamWaitEvent(r->copyStream, r->copyEvent, 0));
         }
-        PT_CHECK(r, r->copier->beginUpload(first, 2, s));
-        PT_CHECK(r, r->copier->finish());
-        PT_CHECK(r, r->copier->beginUpload(second, 2, beside ? r->copyStream : s));
+        PT_CHECK(r, uploading.upload(first, 2, s));
+        PT_CHECK(r, uploading.finish());
+        PT_CHECK(r, uploading.upload(second, 2, beside ? r->copyStream : s));
         if (!beside) {
-            PT_CHECK(r, r->copier->finish());
+            PT_CHECK(r, uploading.finish());
         }
     }
     {
-        const int st = finishScene(r, sl, n, beside);
+        const int st = finishScene(r, sl, n, beside ? &uploading : nullptr);
         if (st != PT_OK) {
             if (beside) {
-                r->copier->finish(); // (the caller's arrays are not read after the call)
+                uploading.finish(); // (the caller's arrays are not read after the call)
                 cudaStreamSynchronize(r->copyStream);
             }
             return st;
@@ -1374,7 +1375,12 @@ int pt_create(pt_renderer** out, int device)
         return PT_ERR_CUDA;
     }
     r->stream = r->ownStream;
-    r->copier.reset(new HostCopier(r->device));
+    try {
+        r->copier = HostCopier::of(r->device);
+    } catch (...) {
+        pt_destroy(r);
+        return PT_ERR_OUT_OF_MEMORY;
+    }
     cudaDeviceGetAttribute(&r->smCount, cudaDevAttrMultiProcessorCount, r->device);
     pt_default_params(&r->params);
     r->scenes[0].camera = defaultCamera();
@@ -1979,8 +1985,9 @@ int pt_trace_rays(pt_renderer* r, int n, const float* origins, const float* dirs
     const HostCopier::Piece in[4] = {{dO, const_cast<float*>(origins), 3 * N * sizeof(float)},
         {dD, const_cast<float*>(dirs), 3 * N * sizeof(float)}, {dTmin, const_cast<float*>(tmin), N * sizeof(float)},
         {dTmax, const_cast<float*>(tmax), N * sizeof(float)}};
-    if (e == cudaSuccess) e = r->copier->beginUpload(in, 4, s);
-    const cudaError_t copied = r->copier->finish();
+    HostCopier::Transfer transfer(*r->copier);
+    if (e == cudaSuccess) e = transfer.upload(in, 4, s);
+    const cudaError_t copied = transfer.finish();
     if (e == cudaSuccess) e = copied;
     if (e == cudaSuccess) {
         launchTraceRays(deviceScene(&r->scenes[0]), n, dO, dD, dTmin, dTmax, dHit, dT, dTri, dN, dUv, s, dOverflow);
@@ -1999,8 +2006,8 @@ int pt_trace_rays(pt_renderer* r, int n, const float* origins, const float* dirs
     give(dN, normal, 3 * N * sizeof(float));
     give(dUv, uv, 2 * N * sizeof(float));
     if (e == cudaSuccess) e = cudaMemcpyAsync(&overflow, dOverflow, sizeof(overflow), cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = r->copier->beginDownload(out, pieces, s);
-    const cudaError_t landed = r->copier->finish();
+    if (e == cudaSuccess) e = transfer.download(out, pieces, s);
+    const cudaError_t landed = transfer.finish();
     if (e == cudaSuccess) e = landed;
     const cudaError_t e2 = cudaStreamSynchronize(s);
     if (e == cudaSuccess) {

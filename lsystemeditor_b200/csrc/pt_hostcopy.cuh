@@ -9,10 +9,13 @@
 // build) 11.6 -> 4.5 ms, 1M ray queries (32 MB in, 29 MB out) 8.2 -> 5.0 ms; a 3 MB
 // image gradient, still in the caller's cache, 0.5 ms slower.
 //
-// One copier belongs to one renderer: the threads, 8 MB of pinned memory and
-// the events are made when its transfers are worth it and given back with it.
+// A process has one copier per device, whatever the number of its renderers: the
+// three threads, 8 MB of pinned memory and the events are made when transfers are
+// worth it and given back with the last renderer.  It takes one transfer at a
+// time, from any thread; a transfer that finds it taken copies plainly, so
+// renderers never wait for one another's streams.
 // A process forked off has none of the threads: there the copier copies plainly
-// and is left alone when its owner goes (a condition variable that vanished
+// and is left alone when its renderers go (a condition variable that vanished
 // threads wait on cannot be destroyed).
 #pragma once
 
@@ -22,6 +25,7 @@
 #include <atomic>
 #include <condition_variable>
 #include <cstring>
+#include <map>
 #include <memory>
 #include <mutex>
 #include <thread>
@@ -39,22 +43,28 @@ public:
         size_t bytes;
     };
 
-    struct Deleter {
-        void operator()(HostCopier* c) const
-        {
-            if (!c->forked()) {
-                delete c;
-            }
+    // The copier of a device.
+    static std::shared_ptr<HostCopier> of(int device)
+    {
+        static std::mutex& lock = *new std::mutex; // (outlive every renderer)
+        static std::map<int, std::weak_ptr<HostCopier>>& live = *new std::map<int, std::weak_ptr<HostCopier>>;
+        std::lock_guard<std::mutex> hold(lock);
+        std::shared_ptr<HostCopier> c = live[device].lock();
+        if (c == nullptr || c->forked()) {
+            c.reset(new HostCopier(device), [](HostCopier* p) {
+                if (!p->forked()) {
+                    delete p;
+                }
+            });
+            live[device] = c;
         }
-    };
-    using Owner = std::unique_ptr<HostCopier, Deleter>;
+        return c;
+    }
 
-    explicit HostCopier(int device) : device_(device) {}
     HostCopier(const HostCopier&) = delete;
     HostCopier& operator=(const HostCopier&) = delete;
     ~HostCopier()
     {
-        finish();
         {
             std::lock_guard<std::mutex> lock(mutex_);
             stop_ = true;
@@ -76,26 +86,78 @@ public:
         return total >= kBesideBytes;
     }
 
-    // Starts copying the pieces to the device on stream s; the sources may be
-    // changed, and work that reads the copies be put on s, after finish().
-    // Transfers too small to gain, from memory that is not pageable or on a
-    // stream that cannot be shared with the workers are enqueued at once.
-    cudaError_t beginUpload(const Piece* p, size_t n, cudaStream_t s) { return begin(p, n, s, true); }
-    // Copies the pieces from the device once the work on s is done; the data is
-    // there after finish().
-    cudaError_t beginDownload(const Piece* p, size_t n, cudaStream_t s) { return begin(p, n, s, false); }
+    // One transfer, ended by finish() or with the object.
+    class Transfer {
+    public:
+        explicit Transfer(HostCopier& c) : c_(c) {}
+        Transfer(const Transfer&) = delete;
+        Transfer& operator=(const Transfer&) = delete;
+        ~Transfer() { finish(); }
 
-    cudaError_t finish()
-    {
-        if (!running_ || forked()) {
-            return cudaSuccess;
+        // Starts copying the pieces to the device on stream s; the sources may be
+        // changed, and work that reads the copies be put on s, after finish().
+        // Transfers too small to gain, from memory that is not pageable or on a
+        // stream that cannot be shared with the workers are enqueued at once.
+        cudaError_t upload(const Piece* p, size_t n, cudaStream_t s) { return begin(p, n, s, true); }
+        // Copies the pieces from the device once the work on s is done; the data is
+        // there after finish().
+        cudaError_t download(const Piece* p, size_t n, cudaStream_t s) { return begin(p, n, s, false); }
+
+        cudaError_t finish()
+        {
+            if (!hold_.owns_lock()) {
+                return cudaSuccess;
+            }
+            const cudaError_t e = c_.wait();
+            hold_.unlock();
+            return e;
         }
-        work(0);
-        std::unique_lock<std::mutex> lock(mutex_);
-        done_.wait(lock, [this] { return busy_ == 0; });
-        running_ = false;
-        return static_cast<cudaError_t>(error_.load());
-    }
+
+    private:
+        cudaError_t begin(const Piece* p, size_t n, cudaStream_t s, bool up)
+        {
+            cudaError_t e = finish();
+            size_t total = 0;
+            bool staged = s != cudaStreamPerThread && !c_.forked();
+            for (size_t i = 0; i < n && e == cudaSuccess; ++i) {
+                total += p[i].bytes;
+                cudaPointerAttributes a{};
+                if (p[i].bytes > 0 && cudaPointerGetAttributes(&a, p[i].host) == cudaSuccess) {
+                    staged = staged && a.type == cudaMemoryTypeUnregistered;
+                } else {
+                    cudaGetLastError();
+                }
+            }
+            cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+            staged = staged && total >= kMinBytes && cudaStreamIsCapturing(s, &cs) == cudaSuccess &&
+                cs == cudaStreamCaptureStatusNone && e == cudaSuccess;
+            if (staged) {
+                hold_ = std::unique_lock<std::mutex>(c_.use_, std::try_to_lock);
+                if (hold_.owns_lock()) {
+                    if (c_.plain_ < kWorthBytes) {
+                        c_.plain_ += total;
+                    } else if (c_.ready()) {
+                        c_.start(p, n, s, up);
+                        return cudaSuccess;
+                    }
+                    hold_.unlock();
+                }
+            }
+            for (size_t i = 0; i < n && e == cudaSuccess; ++i) {
+                if (p[i].bytes > 0) {
+                    e = up ? cudaMemcpyAsync(p[i].device, p[i].host, p[i].bytes, cudaMemcpyHostToDevice, s)
+                           : cudaMemcpyAsync(p[i].host, p[i].device, p[i].bytes, cudaMemcpyDeviceToHost, s);
+                }
+            }
+            if (e == cudaSuccess && !up) {
+                e = cudaStreamSynchronize(s);
+            }
+            return e;
+        }
+
+        HostCopier& c_;
+        std::unique_lock<std::mutex> hold_; // of c_.use_, while the copier works on this transfer
+    };
 
 private:
     static constexpr size_t kSlice = 1024u << 10; // (256 KB: 5.8 ms for the mesh above, 512: 4.8, 1024: 4.5)
@@ -113,56 +175,33 @@ private:
 
     bool forked() const { return getpid() != process_; }
 
-    cudaError_t begin(const Piece* p, size_t n, cudaStream_t s, bool up)
+    explicit HostCopier(int device) : device_(device) {}
+
+    void start(const Piece* p, size_t n, cudaStream_t s, bool up)
     {
-        cudaError_t e = finish();
-        size_t total = 0;
-        bool staged = s != cudaStreamPerThread && !forked();
-        for (size_t i = 0; i < n && e == cudaSuccess; ++i) {
-            total += p[i].bytes;
-            cudaPointerAttributes a{};
-            if (p[i].bytes > 0 && cudaPointerGetAttributes(&a, p[i].host) == cudaSuccess) {
-                staged = staged && a.type == cudaMemoryTypeUnregistered;
-            } else {
-                cudaGetLastError();
-            }
+        pieces_.assign(p, p + n);
+        stream_ = s;
+        up_ = up;
+        next_ = 0;
+        error_ = cudaSuccess;
+        slices_ = 0;
+        for (const Piece& q : pieces_) {
+            slices_ += (q.bytes + kSlice - 1) / kSlice;
         }
-        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-        staged = staged && total >= kMinBytes && cudaStreamIsCapturing(s, &cs) == cudaSuccess &&
-            cs == cudaStreamCaptureStatusNone && e == cudaSuccess;
-        if (staged && plain_ < kWorthBytes) {
-            plain_ += total;
-            staged = false;
+        {
+            std::lock_guard<std::mutex> lock(mutex_);
+            busy_ = static_cast<int>(threads_.size());
+            ++turn_;
         }
-        if (staged && ready()) {
-            pieces_.assign(p, p + n);
-            stream_ = s;
-            up_ = up;
-            next_ = 0;
-            error_ = cudaSuccess;
-            slices_ = 0;
-            for (const Piece& q : pieces_) {
-                slices_ += (q.bytes + kSlice - 1) / kSlice;
-            }
-            {
-                std::lock_guard<std::mutex> lock(mutex_);
-                busy_ = static_cast<int>(threads_.size());
-                ++turn_;
-            }
-            running_ = true;
-            wake_.notify_all();
-            return cudaSuccess;
-        }
-        for (size_t i = 0; i < n && e == cudaSuccess; ++i) {
-            if (p[i].bytes > 0) {
-                e = up ? cudaMemcpyAsync(p[i].device, p[i].host, p[i].bytes, cudaMemcpyHostToDevice, s)
-                       : cudaMemcpyAsync(p[i].host, p[i].device, p[i].bytes, cudaMemcpyDeviceToHost, s);
-            }
-        }
-        if (e == cudaSuccess && !up) {
-            e = cudaStreamSynchronize(s);
-        }
-        return e;
+        wake_.notify_all();
+    }
+    // The started transfer's end, with this thread as one of the workers.
+    cudaError_t wait()
+    {
+        work(0);
+        std::unique_lock<std::mutex> lock(mutex_);
+        done_.wait(lock, [this] { return busy_ == 0; });
+        return static_cast<cudaError_t>(error_.load());
     }
 
     // Threads, pinned memory and events (false: they cannot be had; plain copies).
@@ -278,7 +317,7 @@ private:
             char* host = static_cast<char*>(pieces_[k].host) + at;
             char* buffer = buffers + kSlice * b;
             if (up_) {
-                // (the buffer's last copy, of this transfer or an earlier one, has run)
+                // (the buffer's last copy has run)
                 if (!check(cudaEventSynchronize(events[b]))) {
                     break;
                 }
@@ -298,6 +337,12 @@ private:
         for (int r = 0; r < kBuffers; ++r) {
             land((b + r) % kBuffers);
         }
+        if (up_) {
+            // (the next transfer, on another stream perhaps, finds the buffers free)
+            for (int r = 0; r < kBuffers; ++r) {
+                check(cudaEventSynchronize(events[r]));
+            }
+        }
     }
 
     const int device_;
@@ -307,12 +352,12 @@ private:
     char* pinned_ = nullptr;
     cudaEvent_t events_[kBuffers * kWorkers] = {};
     std::vector<std::thread> threads_;
+    std::mutex use_; // held by the transfer that the copier works on
     std::mutex mutex_;
     std::condition_variable wake_, done_;
     bool stop_ = false;
     unsigned long long turn_ = 0; // transfers started
     int busy_ = 0;                // workers that have not finished the current one
-    bool running_ = false;
     // the current transfer
     std::vector<Piece> pieces_;
     cudaStream_t stream_ = nullptr;

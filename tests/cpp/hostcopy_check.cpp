@@ -38,19 +38,21 @@ std::vector<char> bytes(size_t n, uint32_t seed)
 cudaError_t move(HostCopier& c, std::vector<char>& a, std::vector<char>& b, bool up)
 {
     const HostCopier::Piece p = up ? HostCopier::Piece{b.data(), a.data(), a.size()} : HostCopier::Piece{a.data(), b.data(), a.size()};
-    cudaError_t e = up ? c.beginUpload(&p, 1, kStream) : c.beginDownload(&p, 1, kStream);
-    const cudaError_t f = c.finish();
+    HostCopier::Transfer t(c);
+    const cudaError_t e = up ? t.upload(&p, 1, kStream) : t.download(&p, 1, kStream);
+    const cudaError_t f = t.finish();
     return e != cudaSuccess ? e : f;
 }
 
 // A copier whose threads and pinned memory have been made.
-HostCopier::Owner warm()
+std::shared_ptr<HostCopier> warm()
 {
-    HostCopier::Owner c(new HostCopier(0));
+    std::shared_ptr<HostCopier> c = HostCopier::of(0);
     std::vector<char> a(256 * kMb), b(256 * kMb);
+    const int allocs = fake::hostAllocs;
     CHECK(move(*c, a, b, true) == cudaSuccess);
     CHECK(move(*c, a, b, true) == cudaSuccess);
-    CHECK(fake::hostAllocs == 1);
+    CHECK(fake::hostAllocs == allocs + 1);
     return c;
 }
 
@@ -58,7 +60,7 @@ HostCopier::Owner warm()
 // copied plainly: few or small transfers never pay for it.
 void stagingRule()
 {
-    HostCopier::Owner c(new HostCopier(0));
+    std::shared_ptr<HostCopier> c = HostCopier::of(0);
     auto moves = [&](size_t n, int times, bool up) {
         std::vector<char> a = bytes(n, static_cast<uint32_t>(n)), b(n);
         for (int k = 0; k < times; ++k) {
@@ -86,7 +88,7 @@ void stagingRule()
 // A forked child gives the copier back without its threads, and copies plainly.
 void forkedChild()
 {
-    HostCopier::Owner c = warm();
+    std::shared_ptr<HostCopier> c = warm();
     usleep(50000); // (the workers wait for the next transfer)
     const pid_t child = fork();
     if (child == 0) {
@@ -105,6 +107,100 @@ void forkedChild()
     CHECK(fake::hostFrees == 1);
 }
 
+// Sixty-four holders on a device share one set of threads and pinned memory, and
+// the last one gives it back; another device has its own.
+void shared()
+{
+    std::vector<std::shared_ptr<HostCopier>> holders;
+    for (int k = 0; k < 64; ++k) {
+        holders.push_back(HostCopier::of(0));
+        std::vector<char> a = bytes(30 * kMb, static_cast<uint32_t>(k)), b(a.size());
+        CHECK(move(*holders.back(), a, b, k % 2 == 0) == cudaSuccess && a == b);
+    }
+    CHECK(fake::hostAllocs == 1 && fake::hostFrees == 0);
+    CHECK(HostCopier::of(1) != holders[0]);
+    while (holders.size() > 1) {
+        holders.pop_back();
+    }
+    CHECK(fake::hostFrees == 0);
+    holders.clear();
+    CHECK(fake::hostFrees == 1);
+    CHECK(warm() != nullptr);
+    CHECK(fake::hostAllocs == 2 && fake::hostFrees == 2);
+}
+
+// Transfers of several threads at once: one of them is staged, the others are
+// copied plainly without waiting for it.
+void threads()
+{
+    std::shared_ptr<HostCopier> c = warm();
+    std::vector<std::thread> t;
+    for (uint32_t k = 0; k < 6; ++k) {
+        t.emplace_back([k, c] {
+            for (uint32_t i = 0; i < 5; ++i) {
+                std::vector<char> a = bytes((13 + k) * kMb + i, 10 * k + i), b(a.size());
+                CHECK(move(*c, a, b, (k + i) % 2 == 0) == cudaSuccess && a == b);
+            }
+        });
+    }
+    for (std::thread& x : t) {
+        x.join();
+    }
+    std::vector<char> a = bytes(20 * kMb, 1), b(a.size()), d(a.size());
+    const HostCopier::Piece p{b.data(), a.data(), a.size()}, q{d.data(), a.data(), a.size()};
+    HostCopier::Transfer first(*c);
+    CHECK(first.upload(&p, 1, kStream) == cudaSuccess); // (holds the copier until its end)
+    const int before = fake::copies;
+    std::thread([&] {
+        HostCopier::Transfer second(*c);
+        CHECK(second.upload(&q, 1, kStream) == cudaSuccess && second.finish() == cudaSuccess && a == d);
+    }).join();
+    CHECK(first.finish() == cudaSuccess && a == b);
+    CHECK(fake::copies <= before + 21);
+}
+
+// Errors of a copy come out of finish(), and the copier works again afterwards;
+// without pinned memory, from pinned sources and while the stream is captured
+// everything is copied plainly.
+void errorsAndPlainCopies()
+{
+    {
+        fake::hostAllocFails = true;
+        std::shared_ptr<HostCopier> c = HostCopier::of(0);
+        std::vector<char> a = bytes(200 * kMb, 1), b(a.size());
+        for (int k = 0; k < 3; ++k) {
+            std::fill(b.begin(), b.end(), 0);
+            CHECK(move(*c, a, b, true) == cudaSuccess && a == b);
+        }
+        CHECK(fake::hostAllocs == 1 && fake::hostFrees == 0);
+        fake::hostAllocFails = false;
+        fake::hostAllocs = 0;
+    }
+    std::shared_ptr<HostCopier> c = warm();
+    std::vector<char> a = bytes(20 * kMb + 5, 3), b(a.size());
+    for (bool up : {true, false}) {
+        fake::failCopyAt = fake::copies + 7;
+        CHECK(move(*c, a, b, up) == cudaErrorInvalidValue);
+        fake::failCopyAt = -1;
+        std::fill(b.begin(), b.end(), 0);
+        CHECK(move(*c, a, b, up) == cudaSuccess && a == b);
+    }
+    int before = fake::copies;
+    fake::pinned = a.data();
+    CHECK(move(*c, a, b, true) == cudaSuccess && fake::copies == before + 1);
+    fake::pinned = nullptr;
+    fake::capturing = true;
+    CHECK(move(*c, a, b, true) == cudaSuccess && fake::copies == before + 2);
+    fake::capturing = false;
+    {
+        HostCopier::Transfer t(*c); // (ended with the object)
+        const HostCopier::Piece p{b.data(), a.data(), a.size()};
+        std::fill(b.begin(), b.end(), 0);
+        CHECK(t.upload(&p, 1, kStream) == cudaSuccess);
+    }
+    CHECK(a == b);
+}
+
 } // namespace
 
 int main(int argc, char** argv)
@@ -115,6 +211,12 @@ int main(int argc, char** argv)
             forkedChild();
         } else if (name == "staging_rule") {
             stagingRule();
+        } else if (name == "shared") {
+            shared();
+        } else if (name == "threads") {
+            threads();
+        } else if (name == "errors_and_plain_copies") {
+            errorsAndPlainCopies();
         } else {
             std::printf("no check named %s\n", name.c_str());
             ++failures;

@@ -19,7 +19,7 @@ def program(tmp_path_factory):
     return out
 
 
-@pytest.mark.parametrize("name", ["forked_child", "staging_rule"])
+@pytest.mark.parametrize("name", ["forked_child", "staging_rule", "shared", "threads", "errors_and_plain_copies"])
 def test_hostcopy(program, name):
     r = subprocess.run([program, name], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0, f"exit {r.returncode}: {r.stdout}{r.stderr}"
