@@ -208,7 +208,7 @@ struct pt_renderer {
     int previewLevels = 0;
     int previewDone = -1;                 // finest preview level rendered since the last reset
     DevBuf<float4> previewBuf;            // all levels, coarsest first
-    DevBuf<char> queryBuf;                // inputs and results of pt_trace_rays
+    DevBuf<char> queryBuf;                // inputs and results of pt_trace_rays (up to kQueryBytesKept)
     std::shared_ptr<HostCopier> copier;   // staged copies from and to pageable memory (the device's)
     cudaStream_t copyStream = nullptr;    // uploads beside the work on `stream` (made by the first large mesh)
     cudaEvent_t copyEvent = nullptr;      // orders the two
@@ -279,6 +279,10 @@ struct pt_renderer {
 };
 
 namespace {
+
+// A query's buffer is given back above this (1.7M rays: allocating and freeing
+// take 0.7 ms, such a query 9 ms and more).
+constexpr size_t kQueryBytesKept = size_t(128) << 20;
 
 int fail(pt_renderer* r, int code, const char* fmt, ...)
 {
@@ -1960,10 +1964,10 @@ int pt_trace_rays(pt_renderer* r, int n, const float* origins, const float* dirs
     }
     PT_CHECK(r, cudaSetDevice(r->device));
     const size_t N = static_cast<size_t>(n);
-    // one buffer, kept for the next query: inputs 8 floats, outputs 1 byte + 7 words per ray
+    // one buffer, kept for the next query up to a size: inputs 8 floats, outputs 1
+    // byte + 7 words per ray
     const size_t bytes = N * (8 * sizeof(float) + 7 * sizeof(float) + 16);
     if (!r->queryBuf.ensure(bytes + 32)) {
-        cudaGetLastError();
         return fail(r, PT_ERR_OUT_OF_MEMORY, "pt_trace_rays: %d rays do not fit", n);
     }
     char* buf = r->queryBuf.p;
@@ -2017,6 +2021,9 @@ int pt_trace_rays(pt_renderer* r, int n, const float* origins, const float* dirs
         rc = cudaFail(r, e, "pt_trace_rays");
     } else {
         r->stats.stack_overflows += static_cast<int32_t>(overflow);
+    }
+    if (r->queryBuf.n > kQueryBytesKept) {
+        r->queryBuf.release();
     }
     return rc;
 }
