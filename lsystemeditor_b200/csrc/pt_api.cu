@@ -35,7 +35,7 @@ namespace {
 template <class T> struct DevBuf {
     T* p = nullptr;
     size_t n = 0;
-    bool ensure(size_t count)
+    bool ensure(size_t count, cudaError_t* why = nullptr)
     {
         if (count <= n && p != nullptr) {
             return true;
@@ -44,8 +44,12 @@ template <class T> struct DevBuf {
         if (count == 0) {
             count = 1;
         }
-        if (cudaMalloc(&p, count * sizeof(T)) != cudaSuccess) {
+        const cudaError_t e = cudaMalloc(&p, count * sizeof(T));
+        if (e != cudaSuccess) {
             cudaGetLastError(); // (the caller reports it; the next call's launch checks must not find it)
+            if (why != nullptr) {
+                *why = e;
+            }
             p = nullptr;
             n = 0;
             return false;
@@ -1967,8 +1971,9 @@ int pt_trace_rays(pt_renderer* r, int n, const float* origins, const float* dirs
     // one buffer, kept for the next query up to a size: inputs 8 floats, outputs 1
     // byte + 7 words per ray
     const size_t bytes = N * (8 * sizeof(float) + 7 * sizeof(float) + 16);
-    if (!r->queryBuf.ensure(bytes + 32)) {
-        return fail(r, PT_ERR_OUT_OF_MEMORY, "pt_trace_rays: %d rays do not fit", n);
+    cudaError_t why = cudaSuccess;
+    if (!r->queryBuf.ensure(bytes + 32, &why)) {
+        return cudaFail(r, why, "pt_trace_rays: device buffer");
     }
     char* buf = r->queryBuf.p;
     // traversal stack overflows of this query (pt_stats.stack_overflows)
