@@ -1303,9 +1303,10 @@ int shadowGrid(const pt_renderer* r, bool count, bool inst)
 // The graphs of four bounce iterations for this launch configuration
 // (captured on first use; false: run without graphs, e.g. when the caller's
 // stream is itself being captured).
-bool ensureBounceGraphs(pt_renderer* r, const LaunchCtx* c, bool inst, int nw)
+bool ensureBounceGraphs(pt_renderer* r, const LaunchCtx* c, bool inst, bool multi, int nw)
 {
-    const unsigned long long key[6] = {reinterpret_cast<unsigned long long>(c), static_cast<unsigned long long>(r->gridExtend),
+    const unsigned long long key[6] = {reinterpret_cast<unsigned long long>(c),
+        static_cast<unsigned long long>(r->gridExtend),
         static_cast<unsigned long long>(r->gridShade) | (static_cast<unsigned long long>(r->gridExtendLaneInst) << 16) |
             (static_cast<unsigned long long>(r->gridShadowLaneInst) << 32),
         static_cast<unsigned long long>(r->gridShadow),
@@ -1313,7 +1314,7 @@ bool ensureBounceGraphs(pt_renderer* r, const LaunchCtx* c, bool inst, int nw)
             (static_cast<unsigned long long>(r->extendLane ? 1 : 0) << 8) |
             (static_cast<unsigned long long>(r->gridExtendLane) << 9) |
             (static_cast<unsigned long long>(r->gridShadowLane) << 22) |
-            (static_cast<unsigned long long>(r->scenes.size() > 1 ? 1 : 0) << 62),
+            (static_cast<unsigned long long>(multi ? 1 : 0) << 62),
         reinterpret_cast<unsigned long long>(r->stream)};
     if (r->bounceGraph[0] != nullptr && std::equal(key, key + 6, r->bounceKey)) {
         return true;
@@ -1332,9 +1333,9 @@ bool ensureBounceGraphs(pt_renderer* r, const LaunchCtx* c, bool inst, int nw)
         }
         int sel = 0;
         for (int it = 0; it < 4; ++it) {
-            launchExtend(c, sel, g == 0 && it == 0, it, extendGrid(r, false, inst), false, inst, r->extendLane, r->scenes.size() > 1, s);
+            launchExtend(c, sel, g == 0 && it == 0, it, extendGrid(r, false, inst), false, inst, r->extendLane, multi, s);
             launchShade(c, sel, it, g == 0 && it == 0, shadeGrid(r, nw), nw, s);
-            launchShadow(c, it, shadowGrid(r, false, inst), false, inst, r->extendLane, r->scenes.size() > 1, s);
+            launchShadow(c, it, shadowGrid(r, false, inst), false, inst, r->extendLane, multi, s);
             launchFinalize(c, sel, r->gridShadow, nw, slotOrdered(r), s);
             sel ^= 1;
         }
@@ -1698,6 +1699,7 @@ int pt_render(pt_renderer* r, int waves)
             return st;
         }
     }
+    const bool multi = r->scenes.size() > 1;
     bool inst = false;
     for (const SceneSlot& sl : r->scenes) {
         inst = inst || sl.instanceCount > 0;
@@ -1738,10 +1740,6 @@ int pt_render(pt_renderer* r, int waves)
         }
         const long long jobs = static_cast<long long>(active) * B;
         const int slots = static_cast<int>(std::min<long long>(std::min(r->capacity, r->capacityWanted), jobs));
-        r->hbatch.jobs = static_cast<unsigned long long>(jobs);
-        // generations: no slot takes a second job; each generation of `slots`
-        // jobs drains before the next one starts
-        r->hbatch.nextJob = static_cast<unsigned long long>(PT_PATH_GENERATIONS ? jobs : slots);
         r->hbatch.activeCount = active;
         r->hbatch.waveBase = static_cast<uint32_t>(r->wavesDone);
         r->hbatch.slotCount = slots;
@@ -1750,10 +1748,11 @@ int pt_render(pt_renderer* r, int waves)
         if (c == nullptr) {
             return fail(r, PT_ERR_CUDA, "launch context upload failed");
         }
-        if (r->scenes.size() > 1) {
+        if (multi) {
             launchSceneJobs(c, static_cast<int>(r->scenes.size()), B, s);
             ++launches;
         }
+        // each generation of `slots` jobs drains before the next one starts
         for (long long jobOffset = 0; jobOffset < jobs; jobOffset += slots) {
             const int genCount = static_cast<int>(std::min<long long>(slots, jobs - jobOffset));
             {
@@ -1761,12 +1760,11 @@ int pt_render(pt_renderer* r, int waves)
                 launchGenerate(c, genCount, 0, nw, s, static_cast<unsigned long long>(jobOffset));
             }
             ++launches;
-            // Every live path advances one bounce per iteration and a finished path's
-            // slot takes the next job, so iterations <= bounce-steps / slots + drain.
-            const long long maxIters =
-                (jobs * (maxDepthEff + 1) + slots - 1) / std::max(slots, 1) + maxDepthEff + 8;
+            // Every live path advances one bounce per iteration; the queue's length is
+            // looked at after every fourth.
+            const long long maxIters = static_cast<long long>(maxDepthEff) + 8;
             int sel = 0;
-            const bool graphs = r->useGraphs && r->profileFlags == 0 && ensureBounceGraphs(r, c, inst, nw);
+            const bool graphs = r->useGraphs && r->profileFlags == 0 && ensureBounceGraphs(r, c, inst, multi, nw);
             for (long long it = 0; graphs; it += 4) {
                 // the same four iterations as below, replayed from a graph: sel is 0
                 // again after four, and the kernels use only the parity of `iter`
@@ -1774,7 +1772,7 @@ int pt_render(pt_renderer* r, int waves)
                     return fail(r, PT_ERR_INTERNAL, "path queue did not drain after %lld iterations", it);
                 }
                 PT_CHECK(r, cudaGraphLaunch(r->bounceGraph[it == 0 ? 0 : 1], s));
-                launches += 4 * (2 + extendKernels(false, inst, r->extendLane) + finalizeKernels(slotOrdered(r)));
+                launches += 4 * (3 + extendKernels(false, inst, r->extendLane));
                 r->profile.launches_extend += 4;
                 r->profile.launches_shadow += 4;
                 unsigned int live = 0;
@@ -1791,7 +1789,8 @@ int pt_render(pt_renderer* r, int waves)
                 const int iter = static_cast<int>(it & 0x7fffffff);
                 {
                     StageTimer tm(r, kExtend);
-                    launchExtend(c, sel, it == 0, iter, extendGrid(r, countVisits, inst), countVisits, inst, r->extendLane, r->scenes.size() > 1, s);
+                    launchExtend(c, sel, it == 0, iter, extendGrid(r, countVisits, inst), countVisits, inst, r->extendLane,
+                        multi, s);
                 }
                 {
                     StageTimer tm(r, kShade);
@@ -1799,27 +1798,25 @@ int pt_render(pt_renderer* r, int waves)
                 }
                 {
                     StageTimer tm(r, kShadow);
-                    launchShadow(c, iter, shadowGrid(r, countVisits, inst), countVisits, inst, r->extendLane, r->scenes.size() > 1, s);
+                    launchShadow(c, iter, shadowGrid(r, countVisits, inst), countVisits, inst, r->extendLane, multi, s);
                 }
                 {
                     StageTimer tm(r, kFinalize);
                     launchFinalize(c, sel, r->gridShadow, nw, slotOrdered(r), s);
                 }
-                launches += 2 + extendKernels(countVisits, inst, r->extendLane) + finalizeKernels(slotOrdered(r));
+                launches += 3 + extendKernels(countVisits, inst, r->extendLane);
                 r->profile.launches_extend += 1;
                 r->profile.launches_shadow += 1;
                 sel ^= 1;
                 if ((it & 3) == 3) {
                     unsigned int live = 0;
-                    PT_CHECK(r, cudaMemcpyAsync(&live, r->qCounts.p + sel, sizeof(unsigned int), cudaMemcpyDeviceToHost, s));
+                    PT_CHECK(r,
+                        cudaMemcpyAsync(&live, r->qCounts.p + sel, sizeof(unsigned int), cudaMemcpyDeviceToHost, s));
                     PT_CHECK(r, cudaStreamSynchronize(s));
                     if (live == 0) {
                         break;
                     }
                 }
-            }
-            if (!PT_PATH_GENERATIONS) {
-                break; // one pass: finished paths' slots took the batch's later jobs
             }
         }
         PT_CHECK(r, cudaGetLastError());
@@ -2091,8 +2088,8 @@ int pt_set_tuning(pt_renderer* r, int path_capacity, int blocks_per_sm)
         r->gridShadow = r->smCount * std::max(bsh, 1);
         r->gridExtendLane = r->smCount * extendLaneOccupancy();
         r->gridShadowLane = r->smCount * shadowLaneOccupancy();
-    r->gridExtendLaneInst = r->smCount * extendLaneInstOccupancy();
-    r->gridShadowLaneInst = r->smCount * shadowLaneInstOccupancy();
+        r->gridExtendLaneInst = r->smCount * extendLaneInstOccupancy();
+        r->gridShadowLaneInst = r->smCount * shadowLaneInstOccupancy();
     }
     return PT_OK;
 }

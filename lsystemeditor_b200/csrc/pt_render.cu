@@ -573,19 +573,9 @@ template <int NW> __device__ __forceinline__ void initPath(const LaunchCtx& c, u
     c.paths.orig[i] = make_float4(ro.x, ro.y, ro.z, 0.0f);
     c.paths.dir[i] = make_float4(rd.x, rd.y, rd.z, 0.0f);
     // The throughput, radiance, depth and next-event flags of a path at depth 0
-    // are 1, 0, 0 and clear: with path generations a whole launch is at depth 0
+    // are 1, 0, 0 and clear: the whole first launch of a generation is at depth 0
     // and they are not stored (generation is bound by its writes: 16.7M paths
     // 329 -> 281 us).
-#if !PT_PATH_GENERATIONS
-    c.paths.thr[i] = make_float4(1.0f, 1.0f, 1.0f, 1.0f);
-    if constexpr (NW == 0) {
-        c.paths.rad[i] = make_float4(0.0f, 0.0f, 0.0f, __int_as_float(0));
-    } else {
-        depthEta(c)[i] = make_float2(__int_as_float(0), 1.0f);
-    }
-    c.paths.visEnv[i] = 0;
-    c.paths.visEmis[i] = 0;
-#endif
     if constexpr (NW > 0) {
         c.paths.hero[i] = spectral::heroU(seed);
     }
@@ -600,33 +590,6 @@ __device__ __forceinline__ void queueNext(const LaunchCtx& c, uint32_t i, unsign
     } else {
         const uint32_t s = warpPush(nextCount);
         nextQueue[s] = i;
-    }
-}
-
-// A terminated path's slot takes the batch's next job, if any, and joins the
-// next extend queue: launches stay full until the batch drains.
-template <int NW>
-__device__ __forceinline__ void recyclePath(const LaunchCtx& c, uint32_t i, unsigned int* nextCount, uint32_t* nextQueue)
-{
-#if PT_PATH_GENERATIONS
-    // (generations: a finished path's slot stays empty until the next
-    // generation; the batch's job counter is not touched per path)
-    (void)c;
-    (void)i;
-    (void)nextCount;
-    (void)nextQueue;
-    return;
-#endif
-    cg::coalesced_group g = cg::coalesced_threads();
-    unsigned long long base = 0;
-    if (g.thread_rank() == 0) {
-        base = atomicAdd(&c.q.batch->nextJob, static_cast<unsigned long long>(g.size()));
-    }
-    base = g.shfl(base, 0);
-    const unsigned long long j = base + g.thread_rank();
-    if (j < c.q.batch->jobs) {
-        initPath<NW>(c, i, j);
-        queueNext(c, i, nextCount, nextQueue);
     }
 }
 
@@ -1059,9 +1022,7 @@ __device__ __forceinline__ void listMarked(const LaunchCtx& c, int sel)
 
 // A path whose ray left the scene: previous bounce's NEE, then the
 // environment / background term (PathIntegratorRandCore.h:215-216, 338-346).
-template <int NW>
-__device__ __forceinline__ void shadeMiss(const LaunchCtx& c, uint32_t i, bool fresh, unsigned int* nextCount,
-    uint32_t* nextQueue)
+template <int NW> __device__ __forceinline__ void shadeMiss(const LaunchCtx& c, uint32_t i, bool fresh)
 {
     const Waves<NW> wv = pathWaves<NW>(c, i);
     const float4 d4 = c.paths.dir[i];
@@ -1097,7 +1058,6 @@ __device__ __forceinline__ void shadeMiss(const LaunchCtx& c, uint32_t i, bool f
         }
     }
     writeSample<NW>(c, i, L, wv);
-    recyclePath<NW>(c, i, nextCount, nextQueue);
 }
 
 // Shading of the paths that hit a triangle, then of those that left the scene.
@@ -1404,8 +1364,7 @@ __global__ void __launch_bounds__(kShadeThreads, PT_SHADE_MIN_BLOCKS)
             const float u1 = curand_uniform(&st);
             const float u2 = curand_uniform(&st);
             const BsdfSample smp = bsdfSample(cx, u1, u2);
-            if (!smp.valid || smp.pdf <= kMinPdf) {
-            } else {
+            if (smp.valid && !(smp.pdf <= kMinPdf)) {
                 const Col<NW> f = evalCol<NW>(cx, smp.dir, rho, scatterCoef, wv);
                 T = throughCol<NW>(T, cx, smp, f, rho);
                 if (smp.sss && smp.sssSteps > 0) {
@@ -1433,8 +1392,7 @@ __global__ void __launch_bounds__(kShadeThreads, PT_SHADE_MIN_BLOCKS)
                     }
                 }
                 const float tl = pathWeight<NW>(T);
-                if (!isfinite(tl) || tl <= 0.0f || tl > 1.0e8f) {
-                    } else {
+                if (isfinite(tl) && !(tl <= 0.0f) && !(tl > 1.0e8f)) {
                     bool survive = true;
                     if (depth >= c.rrMinDepth) {
                         const float surv = fmin2(0.95f, fmax2(tl, 0.05f));
@@ -1444,8 +1402,7 @@ __global__ void __launch_bounds__(kShadeThreads, PT_SHADE_MIN_BLOCKS)
                             T = cscl(T, 1.0f / surv);
                         }
                     }
-                    if (!survive) {
-                            } else {
+                    if (survive) {
                         eta = smp.nextEta;
                         const float bias = fmax2(1.0e-4f, 1.0e-3f * t);
                         const float sign = dot3(n, smp.dir) >= 0.0f ? 1.0f : -1.0f;
@@ -1477,7 +1434,6 @@ __global__ void __launch_bounds__(kShadeThreads, PT_SHADE_MIN_BLOCKS)
                     c.q.finish[s] = i;
                 } else {
                     writeSample<NW>(c, i, L, wv);
-                    recyclePath<NW>(c, i, nextCount, nextQueue);
                 }
             } else {
                 if (live) {
@@ -1502,7 +1458,6 @@ __global__ void __launch_bounds__(kShadeThreads, PT_SHADE_MIN_BLOCKS)
                     }
                 } else {
                     writeSample<NW>(c, i, L, wv);
-                    recyclePath<NW>(c, i, nextCount, nextQueue);
                 }
                 c.paths.visEnv[i] = 0;
                 c.paths.visEmis[i] = 0;
@@ -1512,7 +1467,7 @@ __global__ void __launch_bounds__(kShadeThreads, PT_SHADE_MIN_BLOCKS)
     const unsigned int misses = c.q.counts[4 + 2 * (iter & 1)];
     for (unsigned int k = (gridDim.x - 1u - blockIdx.x) * blockDim.x + threadIdx.x; k < misses;
          k += gridDim.x * blockDim.x) {
-        shadeMiss<NW>(c, c.q.missQueue[k], fresh, nextCount, nextQueue);
+        shadeMiss<NW>(c, c.q.missQueue[k], fresh);
     }
 }
 
@@ -1557,15 +1512,13 @@ __global__ void __launch_bounds__(256, 4) k_shadow(const LaunchCtx* __restrict__
 }
 
 // Paths that terminated while their NEE shadow rays were in flight; in
-// slot-ordered mode also the next bounce's extend queue (List; with path
-// generations nothing here marks a slot).
+// slot-ordered mode also the next bounce's extend queue (List; nothing here
+// marks a slot).
 template <int NW, bool List>
 __global__ void __launch_bounds__(kListThreads) k_finalize(const LaunchCtx* __restrict__ cp, int sel)
 {
     const LaunchCtx& c = *cp;
     const unsigned int count = c.q.counts[3];
-    unsigned int* nextCount = &c.q.counts[sel ^ 1];
-    uint32_t* nextQueue = c.q.extend[sel ^ 1];
     for (unsigned int k = blockIdx.x * blockDim.x + threadIdx.x; k < count; k += gridDim.x * blockDim.x) {
         const uint32_t i = c.q.finish[k];
         const Waves<NW> wv = pathWaves<NW>(c, i);
@@ -1577,14 +1530,11 @@ __global__ void __launch_bounds__(kListThreads) k_finalize(const LaunchCtx* __re
             L = cadd(L, pendingEmis<NW>(c, i));
         }
         writeSample<NW>(c, i, L, wv);
-        recyclePath<NW>(c, i, nextCount, nextQueue);
-    }    if constexpr (List) {
+    }
+    if constexpr (List) {
         listMarked(c, sel);
     }
 }
-#if !PT_PATH_GENERATIONS
-__global__ void __launch_bounds__(kListThreads) k_next_queue(const LaunchCtx* __restrict__ cp, int sel) { listMarked(*cp, sel); }
-#endif
 
 // Per pixel: fold the batch's samples in sample order (PathTracer.cu:232-272).
 // activeCount[1] counts the pixels that go on (KeepActive), so that the list is
@@ -1906,13 +1856,12 @@ int shadowLaneInstOccupancy()
 }
 void launchShade(const LaunchCtx* c, int sel, int iter, bool first, int grid, int nw, cudaStream_t s)
 {
-    const bool fresh = first && PT_PATH_GENERATIONS != 0;
     if (nw == 8) {
-        k_shade<8><<<grid, kShadeThreads, 0, s>>>(c, sel, iter, fresh);
+        k_shade<8><<<grid, kShadeThreads, 0, s>>>(c, sel, iter, first);
     } else if (nw == 4) {
-        k_shade<4><<<grid, kShadeThreads, 0, s>>>(c, sel, iter, fresh);
+        k_shade<4><<<grid, kShadeThreads, 0, s>>>(c, sel, iter, first);
     } else {
-        k_shade<0><<<grid, kShadeThreads, 0, s>>>(c, sel, iter, fresh);
+        k_shade<0><<<grid, kShadeThreads, 0, s>>>(c, sel, iter, first);
     }
 }
 void launchShadow(const LaunchCtx* c, int iter, int grid, bool count, bool inst, bool lane, bool multi, cudaStream_t s)
@@ -1970,18 +1919,11 @@ void stageOccupancy(int& extendBlocks, int& shadeBlocks, int& shadowBlocks)
 namespace {
 template <int NW> void finalize(const LaunchCtx* c, int sel, int grid, bool list, cudaStream_t s)
 {
-#if PT_PATH_GENERATIONS
     if (list) {
         k_finalize<NW, true><<<grid, kListThreads, 0, s>>>(c, sel);
-        return;
+    } else {
+        k_finalize<NW, false><<<grid, kListThreads, 0, s>>>(c, sel);
     }
-#endif
-    k_finalize<NW, false><<<grid, kListThreads, 0, s>>>(c, sel);
-#if !PT_PATH_GENERATIONS
-    if (list) {
-        k_next_queue<<<grid, kListThreads, 0, s>>>(c, sel);
-    }
-#endif
 }
 } // namespace
 void launchFinalize(const LaunchCtx* c, int sel, int grid, int nw, bool list, cudaStream_t s)
@@ -1994,7 +1936,6 @@ void launchFinalize(const LaunchCtx* c, int sel, int grid, int nw, bool list, cu
         finalize<0>(c, sel, grid, list, s);
     }
 }
-int finalizeKernels(bool list) { return list && !PT_PATH_GENERATIONS ? 2 : 1; }
 void launchAccumulate(const LaunchCtx* c, int activeCount, int batch, cudaStream_t s)
 {
     k_accumulate<<<gridFor(activeCount, kAccumulateThreads), kAccumulateThreads, 0, s>>>(c, activeCount, batch);

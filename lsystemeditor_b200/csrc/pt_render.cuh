@@ -3,17 +3,6 @@
 
 #include "pt_common.cuh"
 
-#ifndef PT_PATH_GENERATIONS
-// Jobs of a batch run in generations of the slot count, each drained before
-// the next, instead of refilling each finished path's slot with the next job:
-// the launches of a generation hold paths of the same depth (camera rays
-// together, then first bounces, ...).  Same images; plain-large 1106 -> 1068
-// ms per frame, a 1920x1080 forest view 10.59 -> 10.47 s, the 64-tree batch
-// 20.71 -> 18.37 s; and 1068 -> 1035 ms once finished paths stopped claiming
-// jobs from the batch's counter.
-#define PT_PATH_GENERATIONS 1
-#endif
-
 namespace pt {
 
 // Structure-of-arrays path state, capacity `capacity` paths.
@@ -46,10 +35,14 @@ struct PathSoA {
 };
 
 // Current batch of (pixel, sample) jobs (device memory; written by the host at
-// batch start, nextJob advanced by the kernels that recycle path slots).
+// batch start).  Jobs run in generations of the slot count, each drained before
+// the next, so that the launches of a generation hold paths of the same depth
+// (camera rays together, then first bounces, ...): against refilling each
+// finished path's slot with the next job, 1106 -> 1068 ms per frame of 972k
+// triangles at 1024^2, a 1920x1080 forest view 10.59 -> 10.47 s, 64 trees 20.71 ->
+// 18.37 s; and 1068 -> 1035 ms once finished paths no longer claimed jobs from
+// the batch's counter.
 struct BatchInfo {
-    unsigned long long jobs;     // activeCount x waves in this batch
-    unsigned long long nextJob;  // first job not yet handed to a path slot
     int activeCount;
     uint32_t waveBase;
     int slotCount;               // path slots in use in this batch
@@ -184,8 +177,6 @@ void launchShade(const LaunchCtx* d, int sel, int iter, bool first, int grid, in
 void launchShadow(const LaunchCtx* d, int iter, int grid, bool count, bool inst, bool lane, bool multi, cudaStream_t s);
 // list: slot-ordered mode, the next bounce's extend queue from the marked slots.
 void launchFinalize(const LaunchCtx* d, int sel, int grid, int nw, bool list, cudaStream_t s);
-// Kernels one launchFinalize call launches.
-int finalizeKernels(bool list);
 void launchAccumulate(const LaunchCtx* d, int activeCount, int batch, cudaStream_t s);
 // Stable compaction of the active list (pixels neither converged nor at the
 // sample cap), so that the list stays sorted by pixel and thereby by scene.
