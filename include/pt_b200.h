@@ -269,7 +269,8 @@ int pt_get_profile(const pt_renderer* r, pt_profile* out);
 int pt_set_tuning(pt_renderer* r, int path_capacity, int blocks_per_sm);
 
 /* Closest-hit and shadow-ray scheduling (no reference counterpart; images are
- * identical in every mode).  AUTO and LANE: whole-warp traversal with ray
+ * identical in every mode, but for which of several surfaces that overlap in
+ * one plane a ray returns).  AUTO and LANE: whole-warp traversal with ray
  * replacement (closest hit and shadow rays; two-level traversal in instanced
  * scenes) and a slot-ordered next-bounce queue.  WARP: one warp per 32 queued
  * rays, each lane on its own. */
@@ -540,7 +541,7 @@ int pt_reset_region(pt_renderer* r);
  * normals and uvs may be NULL: without normals the reported normal is the
  * triangle's geometric normal facing the ray, without uvs the uv is 0; results
  * as in pt_trace_rays); work runs on `stream` (NULL = default stream) of the
- * current device.  The BVH build waits for `stream` once per tree level, so
+ * current device.  The BVH build waits for `stream` once per four tree levels, so
  * the call blocks the host until the build is done and returns with the
  * traversal enqueued.  All temporaries live in one 8 MiB device array,
  * reserved on a GPU when the library's module is first loaded there (at the

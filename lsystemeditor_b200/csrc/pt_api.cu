@@ -1706,7 +1706,7 @@ int pt_render(pt_renderer* r, int waves)
     }
     // The whole-warp traversal, its routing and its slot-ordered queues are the
     // better form for every size of scene (2.4k triangles, 641x359, 16 spp: closest
-    // hit 7.0 -> 3.7 ms; 20k triangles, 96x64, one sample: even).
+    // hit 7.0 -> 3.3 ms; 20k triangles, 96x64, one sample: even).
     r->extendLane = r->extendMode != PT_EXTEND_MODE_WARP;
     const int nw = r->params.spectral_wavelengths;
     if (nw > 0) {

@@ -179,7 +179,7 @@ int buildBvhInto(const float* dPositions, uint32_t n, const BvhScratch& scratch,
 
 // Builds the compressed 8-wide BVH over n triangles whose positions
 // (9 floats per triangle) are already in device memory. Synchronises the
-// stream once per collapse level. Returns a pt_status code.
+// stream once per four collapse levels. Returns a pt_status code.
 int buildBvh(const float* dPositions, uint32_t n, BvhBuffers& out, cudaStream_t stream, const BvhBuildOptions& opt,
     char* err, size_t errLen);
 

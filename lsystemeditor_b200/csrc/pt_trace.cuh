@@ -11,7 +11,11 @@
 //     neither on the visiting order nor on the BVH's layout -- the parallel
 //     top-down collapse places nodes and leaves in an order that differs
 //     between builds -- so every kernel, and every build of the same scene,
-//     picks the same triangle;
+//     picks the same of the triangles that it tests.  (Which it tests can depend
+//     on the order where two hits are closer together than the box test is
+//     exact, see hitSlack.  The whole-warp kernels keep one order; those with one
+//     ray per lane postpone triangle tests by what the warp's other rays do, and
+//     on overlapping coplanar surfaces may return another of them.);
 //   * a hit is reported only if the final t < tMax;
 //   * quirk Q1: a direction component with |d| <= 1e-8 gets a zero reciprocal
 //     in the reference, which turns every slab test into "does the box contain
@@ -19,8 +23,9 @@
 //     reference's leaves are single triangles with exact bounds, so this is
 //     reproduced independently of the tree by testing only triangles whose
 //     exact bounds contain the origin in the non-degenerate axes (traceQ1).
-// Child boxes are quantised outward, so the tree is conservative; the slab
-// test widens tExit by 2^-21 relative to absorb its own rounding.
+// Child boxes are quantised outward; the slab test widens tExit by 2^-21
+// relative, which covers its rounding for boxes about as far away as the tree
+// is large, not for those right before the origin (hitSlack).
 #pragma once
 
 #include "pt_common.cuh"

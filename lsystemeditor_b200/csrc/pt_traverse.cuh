@@ -30,7 +30,7 @@
 // overlapping coplanar rectangles rendered differently from run to run, in up to
 // 3% of their pixels.  Few rays need it (8 of the 403M of the large frame below,
 // 159 of the 4.9M of a 256^2 frame of 20k triangles whose tubes share their ends:
-// 1.11 -> 1.15 ms; the other timed frames within 1.5%).
+// 1.13 -> 1.16 ms; 1024^2 waves 6.42 -> 6.54; the other timed frames within 0.5%).
 //
 // Why: in a free-running loop (a lane fetched and stepped on its own) 6 of 32
 // lanes worked per executed instruction, a node's triangles were tested one
