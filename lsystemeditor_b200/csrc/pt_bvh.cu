@@ -638,10 +638,15 @@ struct CollapseArgs {
 };
 
 // Smallest exponent e with extent <= 255 * 2^e (extent computed exactly in double).
+// Finite boxes need at most 2^121; an infinite one gets 2^127, so that the biased
+// exponent stays a byte (a larger one would run into the node's child mask).
 __device__ __forceinline__ int quantExp(double extent)
 {
     if (!(extent > 0.0)) {
         return -126;
+    }
+    if (extent > 2.0 * FLT_MAX) {
+        return 127;
     }
     int e;
     frexp(extent / 255.0, &e); // extent/255 in [2^(e-1), 2^e)
